@@ -186,24 +186,26 @@ int sf_set_xpass_slabs(sf_solver* s, int slabs);
  * the other over all levels. The results do not depend on it. */
 int sf_set_xy_bands(sf_solver* s, int bands);
 
-/* Launch tuning of the z solves (no counterpart in the reference): the
- * warps per block of the z solves, 8 or 16 (0: 16 when one block per group
- * of 16 modes leaves SMs idle, else 8). Each warp takes one z-chunk of every
- * Thomas system in z kernels 0 and 1 (sf_set_z_kernel) and two in the
- * default kernel 2, which needs N3 >= 64 for 16 warps (else it takes 8). The
- * results depend on it only through rounding (the chunked solve
- * reassociates the recurrence). */
+/* Launch tuning of the z solves (no counterpart in the reference): 8 or 16
+ * (0: chosen from the grid). In z kernels 0 and 1 (sf_set_z_kernel) the warps
+ * per block, each with one z-chunk of every Thomas system (0: 16 when one
+ * block per group of 16 modes leaves SMs idle, else 8). In the default
+ * kernel 2, 8 asks for blocks of which two share an SM and 16 for blocks of
+ * which one fills it, where the grid has both. The results depend on it only
+ * through rounding (the chunked solve reassociates the recurrence). */
 int sf_set_z_chunks(sf_solver* s, int chunks);
 
 /* Launch tuning of the z pass (no counterpart in the reference): kind 2 (the
- * default) runs it as k_z_step_c, one lane per complex mode in paired FP32
- * instructions and two z-chunks per warp (16 chunks per block; grids with
- * N3 >= 32, else kind 0 runs); kind 0 as k_z_step, one lane per real
+ * default) runs it as k_z_step_f, which solves every field of a group of 8
+ * modes at the same time and keeps the new velocities in shared memory for the
+ * projection (grids with N3 >= 32, else kind 0 runs; grids too tall for its
+ * shared memory, 3D above N3 = 672 and 2D above 824, run k_z_step_c, one field after the
+ * other, one lane per complex mode); kind 0 as k_z_step, one lane per real
  * component and one chunk per warp; kind 1 as k_z_step_tma, k_z_step with
  * each warp's first-sweep inputs brought into shared memory by
  * tensor-memory-accelerator copies and the Thomas intermediates in tensor
  * memory (with 8 z chunks; a wait for its tiles that runs out is reported by
- * sf_synchronize). The three solve the same systems with the same terms; the
+ * sf_synchronize). All solve the same systems with the same terms; the
  * results differ by rounding (the chunk count reassociates the recurrences). */
 int sf_set_z_kernel(sf_solver* s, int kind);
 

@@ -411,15 +411,15 @@ class IMEXRK:
         _check(load_library().sf_set_xpass_kernel(self._h, int(kind)))
 
     def set_z_kernel(self, kind):
-        """z pass: 2 k_z_step_c (default, one lane per complex mode), 0
-        k_z_step, 1 k_z_step_tma (TMA-fed first sweeps); a launch setting
-        (the results change only by rounding)."""
+        """z pass: 2 k_z_step_f (default, every field of a mode group at
+        once), 0 k_z_step, 1 k_z_step_tma (TMA-fed first sweeps); a launch
+        setting (the results change only by rounding)."""
         _check(load_library().sf_set_z_kernel(self._h, int(kind)))
 
     def set_z_chunks(self, chunks):
-        """Warps per block of the z solves (0: automatic, 8 or 16), each with
-        one z-chunk (k_z_step) or two (k_z_step_c); a launch setting (the
-        results change only by rounding)."""
+        """Block size of the z solves (0: automatic; 8 or 16 warps of
+        k_z_step, two blocks or one per SM in the default kernel); a launch
+        setting (the results change only by rounding)."""
         _check(load_library().sf_set_z_chunks(self._h, int(chunks)))
 
     def set_tangent(self, nbase):

@@ -58,6 +58,11 @@ struct StageArgs {
   const float* zc;      // ZC_COUNT x N3
   const float* fa;      // kNumFS x N3 sub-diagonals a_j
   const float* fc;      // kNumFS x N3 super-diagonals c_j
+  // the same rows packed for k_z_step_f, one vector load per level:
+  const float4* zt1;    // 9 x N3 per Crank-Nicolson factor set: d2z lower, diagonal, upper; a_j
+  const float4* zt2;    // N3: ddz (N -> D) lower, diagonal; ReinterpolateFull lower, diagonal
+  const float4* ztq;    // N3: ddz (D -> N) diagonal, upper; the Laplacian's a_j, c_j
+  const float2* zac;    // kNumFS x N3: a_j, c_j
   const float* inv_den; // kNumFS x N3 x Pp, 1/(b_j - a_j C_{j-1}) (FP64-factorised)
   const float* kx;      // K1
   const float* ky;      // K2
@@ -85,7 +90,7 @@ struct StageArgs {
   int xgroups;      // lane groups per x-pass block (0: chosen by the launcher)
   int xkernel;      // 3D nonlinear x pass: 1 level-marching lane groups (k_xmarch), 0 slab blocks (k_xpass)
   int zkernel;      // z pass: 0 k_z_step, 1 k_z_step_tma (inputs by the tensor-memory accelerator),
-                    // 2 k_z_step_c (one lane per complex mode)
+                    // 2 k_z_step_f (every field of a mode group at once)
   const void* zmaps;   // host ZMaps of the solver (k_z_step_tma), or null
   int* zerr;           // device word set by a k_z_step_tma wait that ran out
 };
@@ -134,6 +139,10 @@ int launch_z_step_c(const StageArgs& a, cudaStream_t st);
 int prepare_zstep_c_kernels();
 bool z_step_takes_c(const StageArgs& a);
 int prepare_zstep_tma_kernels();
+// the z pass with all fields of a mode group at once (sf_zstep3.cu)
+bool zstep_f_supported(const Geo& g);
+int launch_z_step_f(const StageArgs& a, cudaStream_t st);
+int prepare_zstep_f_kernels();
 // the 3D nonlinear x pass as level-marching lane groups (sf_xmarch.cu): levels
 // t_lo .. t_hi - 1 of every run and y row
 bool xmarch_supported(const StageArgs& a);

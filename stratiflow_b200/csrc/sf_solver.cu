@@ -42,6 +42,8 @@ struct sf_solver {
   float2 *rold = nullptr, *rnl = nullptr, *qbuf = nullptr, *mixin = nullptr, *mixout = nullptr;
   float* base = nullptr;
   float *zc = nullptr, *fa = nullptr, *fc = nullptr, *inv_den = nullptr;
+  float4* zt = nullptr;          // k_z_step_f's packed rows: zt1 [9][N3], zt2 [N3], ztq [N3], zac
+  std::vector<float> hzc;        // zc, on the host
   float *kx = nullptr, *ky = nullptr, *Ri = nullptr, *Ubar = nullptr, *dBdz = nullptr;
   double *bands = nullptr, *kxd = nullptr, *kyd = nullptr, *red = nullptr;
   float2* tw = nullptr;
@@ -59,7 +61,7 @@ struct sf_solver {
   int zchunks = 0;               // z chunks per z-solve block (sf_set_z_chunks)
   int xgroups = 0;               // lane groups per x-pass block (sf_set_xpass_groups)
   int xkernel = 1;               // 3D nonlinear x pass: 1 level-marching, 0 slab blocks (sf_set_xpass_kernel)
-  int zkernel = 2;               // z pass: 2 k_z_step_c (default), 0 k_z_step, 1 k_z_step_tma (sf_set_z_kernel)
+  int zkernel = 2;               // z pass: 2 k_z_step_f (default), 0 k_z_step, 1 k_z_step_tma (sf_set_z_kernel)
   ZMaps* zmaps = nullptr;        // tensor maps of k_z_step_tma's inputs (null: not supported here)
   int* zerr = nullptr;           // set on the device by a k_z_step_tma wait that ran out
   cudaGraphExec_t graph[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};   // [linear][parity]
@@ -103,7 +105,7 @@ static void free_all(sf_solver* s) {
       if (s->graph[l][p]) cudaGraphExecDestroy(s->graph[l][p]);
   delete s->zmaps;
   s->zmaps = nullptr;
-  void* ptrs[] = {s->zerr, s->amix, s->adir, s->S[0], s->S[1], s->rold, s->rnl, s->qbuf, s->mixin, s->mixout, s->base, s->zc, s->fa,
+  void* ptrs[] = {s->zt, s->zerr, s->amix, s->adir, s->S[0], s->S[1], s->rold, s->rnl, s->qbuf, s->mixin, s->mixout, s->base, s->zc, s->fa,
                   s->fc, s->inv_den, s->kx, s->ky, s->Ri, s->Ubar, s->dBdz, s->bands, s->kxd, s->kyd,
                   s->red, s->tw, s->stage_ref};
   for (void* p : ptrs)
@@ -191,6 +193,23 @@ static int refactor(sf_solver* s) {
   build_rows(s, b6, fa, fc);
   CK(cudaMemcpyAsync(s->fa, fa.data(), sizeof(float) * fa.size(), cudaMemcpyHostToDevice, s->st));
   CK(cudaMemcpyAsync(s->fc, fc.data(), sizeof(float) * fc.size(), cudaMemcpyHostToDevice, s->st));
+  // the packed rows of k_z_step_f; they and fa, fc end after the wait below
+  std::vector<float4> zt((size_t)11 * N + kNumFS * N / 2);
+  {
+    float2* ac = reinterpret_cast<float2*>(zt.data() + (size_t)11 * N);
+    auto z = [&](int r, int j) { return s->hzc[(size_t)r * N + j]; };
+    for (int fs = 0; fs < kNumFS; fs++)
+      for (int j = 0; j < N; j++) {
+        const float aj = fa[(size_t)fs * N + j], cj = fc[(size_t)fs * N + j];
+        ac[(size_t)fs * N + j] = make_float2(aj, cj);
+        const int lo = fs / 3 == 2 ? ZC_D2D_LO : ZC_D2N_LO;
+        if (fs != kFS_Lap) zt[(size_t)fs * N + j] = make_float4(z(lo, j), z(lo + 1, j), z(lo + 2, j), aj);
+        else zt[(size_t)10 * N + j] = make_float4(z(ZC_DDN_DI, j), z(ZC_DDN_UP, j), aj, cj);
+      }
+    for (int j = 0; j < N; j++)
+      zt[(size_t)9 * N + j] = make_float4(z(ZC_DND_LO, j), z(ZC_DND_DI, j), z(ZC_FULL_LO, j), z(ZC_FULL_DI, j));
+  }
+  CK(cudaMemcpyAsync(s->zt, zt.data(), sizeof(float4) * zt.size(), cudaMemcpyHostToDevice, s->st));
   s->launches += launch_factor(s->g, s->bands, s->kxd, s->kyd, s->h[0], s->h[1], s->h[2], s->Re, s->Pr,
                                s->inv_den, s->st);
   CK(cudaGetLastError());
@@ -212,6 +231,10 @@ static StageArgs stage_args(sf_solver* s, int k, int cur, bool linear) {
   a.zc = s->zc;
   a.fa = s->fa;
   a.fc = s->fc;
+  a.zt1 = s->zt;
+  a.zt2 = s->zt + (size_t)9 * s->g.N3;
+  a.ztq = s->zt + (size_t)10 * s->g.N3;
+  a.zac = reinterpret_cast<const float2*>(s->zt + (size_t)11 * s->g.N3);
   a.inv_den = s->inv_den;
   a.kx = s->kx;
   a.ky = s->ky;
@@ -353,6 +376,7 @@ int sf_create(const sf_grid* grid, const sf_flow* flow, double dt, int device, s
   CKC(cudaMalloc(&s->zc, sizeof(float) * ZC_COUNT * N3));
   CKC(cudaMalloc(&s->fa, sizeof(float) * kNumFS * N3));
   CKC(cudaMalloc(&s->fc, sizeof(float) * kNumFS * N3));
+  CKC(cudaMalloc(&s->zt, sizeof(float4) * (11 * N3 + kNumFS * N3 / 2)));
   CKC(cudaMalloc(&s->inv_den, sizeof(float) * kNumFS * g.fblk));
   CKC(cudaMalloc(&s->kx, sizeof(float) * g.K1));
   CKC(cudaMalloc(&s->ky, sizeof(float) * g.K2));
@@ -418,6 +442,7 @@ int sf_create(const sf_grid* grid, const sf_flow* flow, double dt, int device, s
   for (int k = 1; k < N - 1; k++) zc[(size_t)ZC_WZN * N + k] = (float)(z[k + 1] - z[k]);
   for (int k = 2; k < N - 1; k++) zc[(size_t)ZC_WZD * N + k] = (float)(zf[k] - zf[k - 1]);
   CKC(cudaMemcpy(s->bands, b6.data(), sizeof(double) * 6 * N, cudaMemcpyHostToDevice));
+  s->hzc = zc;
   CKC(cudaMemcpy(s->zc, zc.data(), sizeof(float) * zc.size(), cudaMemcpyHostToDevice));
   // ---- Fourier wavenumbers, Differentiation.cpp:113-160 ----
   {
@@ -780,7 +805,7 @@ int sf_profile_names(sf_solver* s, char* buf, size_t len) {
   const bool march = s->xkernel == 1 && !s->tlm && xmarch_supported(stage_args(s, 0, s->cur, false));
   // and the z pass as k_z_step_tma
   const StageArgs a0 = stage_args(s, 0, s->cur, false);
-  const char* zname = z_step_takes_c(a0) ? "k_z_step_c" : (z_step_takes_tma(a0) ? "k_z_step_tma" : "k_z_step");
+  const char* zname = z_step_takes_c(a0) ? (zstep_f_supported(a0.g) ? "k_z_step_f" : "k_z_step_c") : (z_step_takes_tma(a0) ? "k_z_step_tma" : "k_z_step");
   for (int k = 0; k < 3; k++)
     for (int i = 0; i < stage_kernel_count(s->g); i++) {
       if (!out.empty()) out += ",";
