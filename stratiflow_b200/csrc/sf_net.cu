@@ -12,11 +12,14 @@
 //   forward          m = co, n = (b,z),        k = (tap,ci)
 //   backward data    m = ci, n = (b,z),        k = (tap,co)
 //   backward weights m = co, n = (tap,ci),     k = (b,z)
-// issued as tcgen05.mma on 128 x 128 tiles with the accumulator in tensor
-// memory (k_conv_gemm_tc).
+// issued as tcgen05.mma on 128 x 64 tiles with the accumulator in tensor
+// memory, the operands brought in by tensor-map copies (k_conv_gemm_tc).
+#include <cuda.h>
+#include <cudaTypedefs.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <random>
 #include <string>
@@ -33,12 +36,8 @@ constexpr int kTaps = 5, kPad = 2;
 enum GemmMode { G_FWD = 0, G_BWD_DATA = 1, G_BWD_W = 2 };
 
 struct ConvGemm {
-  int mode;
   int B, Z, Cin, Cout;
-  int M, N, K;
-  const __nv_bfloat16* W;    // [Cout][tap][Cin]
-  const __nv_bfloat16* X;    // layer input [B][Z][Cin]
-  const __nv_bfloat16* dP;   // gradient of the pre-activation [B][Z][Cout]
+  int M;                     // rows of C
   const float* bias;         // forward
   float* outF;               // FP32 result (forward output layer, dW)
   __nv_bfloat16* outB;       // BF16 result (activation, dP of the layer below)
@@ -47,46 +46,67 @@ struct ConvGemm {
 };
 
 // ---------------------------------------------------------------- tcgen05 --
-// The implicit GEMMs on the 5th-generation tensor cores: a CTA of four
-// warps computes a 128 x 128 tile of C with tcgen05.mma (kind::f16, BF16 x
-// BF16 -> FP32) issued by one thread, the accumulator in tensor memory (128
-// lanes x 128 FP32 columns), A and B staged in shared memory as 64-wide K
-// slices in the K-major layout with the 128-byte swizzle: each row's 64
-// elements are one 128-byte line whose 16-byte chunk c sits at c ^ (row % 8),
-// 8-row groups 1024 bytes apart (SBO); an instruction's K = 16 is the next 32
-// bytes of every row (the descriptor's start address advances by 32 bytes).
-// The 16-byte operand loads of one row then fill one line without bank
-// conflicts.
-// Two shared-memory stages: the loads of K slice t + 1 overlap the MMAs of
-// slice t, and an mbarrier that the MMAs' commit arrives on frees a stage.
-// Every wait is bounded; a wait that runs out sets *err and the block skips
-// to freeing its tensor memory.
-constexpr int TM = 128, TN = 128, TK = 64, kTcThreads = 128;
-constexpr int kTcStageElems = (TM + TN) * TK;                      // bf16 per stage
-// two stages, plus room to align the first to the swizzle's 1024-byte period
-constexpr size_t kTcSmem = sizeof(__nv_bfloat16) * 2 * kTcStageElems + 1024;
-constexpr long long kTcSpin = 1ll << 26;                           // bounded mbarrier waits
+// The implicit GEMMs on the 5th-generation tensor cores. A CTA of four warps
+// computes a 128 x 64 tile of C: a tile's n are 64 levels of one sample
+// (forward, backward data) or 64 input channels of one tap (backward weights).
+// Every K slice of 64 is one tap's run of 64 channels, or one sample's run of
+// 64 levels, so both operands of a slice are boxes of the tensors as they lie
+// in memory: X and dP as [B][Z][C], W as [Cout][tap][Cin]. Thread 0 brings
+// them in by cp.async.bulk.tensor (levels outside 0..Z-1 and channels past C
+// arrive as zeros: the convolution's padding and the tiles' edges need no
+// code), thread 32 issues tcgen05.mma (kind::f16, BF16 x BF16 -> FP32, M =
+// 128, N = 64, K = 16) with the accumulator in tensor memory, all four warps
+// read it back. A slice's operands lie in shared memory in the 128-byte
+// swizzle, with K contiguous (forward; backward data's dP) or with M or N
+// contiguous (backward data's W, both operands of the weight gradient: the
+// instruction's transpose bits), as the tensors have them.
+//
+// Bound by the operands' way from L2: 24 KB a slice and SM, which takes about
+// 790 cycles on 104 SMs at once (6.1 TB/s over the GPU) against the
+// instructions' 128; four slices in flight per CTA, two CTAs per SM (eight
+// slices measured the same). Measured, 13 samples of 256 levels: 1024 -> 256
+// channels forward 32 us, the 11 GEMMs of one gradient 0.18 ms in 8 launches,
+// where the version that gathered operands through registers took 3.29 ms.
+//
+// The K slices, and the runs of 16 of an instruction within them, go in the
+// order of (tap, channel), one accumulator per tile: a result does not depend
+// on the tiling. Every wait is bounded; one that runs out sets *err, the other
+// waits of the block then give up at once, and the block waits for its copies
+// in flight and frees its tensor memory.
+constexpr int TM = 128, TN = 64, TK = 64, kTcThreads = 128, kTcStages = 4, kMaxLayers = 16;
+constexpr int kTcABytes = TM * TK * 2, kTcBBytes = TN * TK * 2, kTcStageBytes = kTcABytes + kTcBBytes;
+// the stages, and room to align the first to the swizzle's 1024-byte period
+static_assert(TN == TK, "the X and dP maps' boxes serve as N tiles and as K slices");
+constexpr size_t kTcSmem = (size_t)kTcStages * kTcStageBytes + 1024;
+constexpr int kTcSpin = 1 << 22;                                   // bounded mbarrier waits
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-// K-major shared-memory matrix descriptor (sm_100) of the 128-byte swizzle:
-// start address and the byte offsets in 16-byte units (LBO 16 bytes, unused
-// by this layout; SBO 1024 bytes between 8-row groups), descriptor version 1,
-// layout type 2 (SWIZZLE_128B)
-__device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t addr) {
-  return (uint64_t)((addr >> 4) & 0x3FFF) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) |
-         (2ull << 61);
+// shared-memory matrix descriptor (sm_100) of the 128-byte swizzle: start
+// address and the byte offsets in 16-byte units, descriptor version 1, layout
+// type 2 (SWIZZLE_128B). K contiguous: rows of 64 K values, 8-row groups SBO =
+// 1024 bytes apart (LBO unused). M or N contiguous: rows of 64 M or N values,
+// one per k, 8-k groups SBO = 1024 bytes apart, the next 64 M or N values
+// LBO = 8192 bytes on (64 k rows of 128 bytes).
+__device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t addr, bool mn) {
+  return (uint64_t)((addr >> 4) & 0x3FFF) | ((uint64_t)(mn ? 8192 >> 4 : 1) << 16) | ((uint64_t)(1024 >> 4) << 32) |
+         (1ull << 46) | (2ull << 61);
 }
 
-// instruction descriptor of kind::f16: D FP32, A and B BF16, both K-major,
-// N and M of the instruction
-__host__ __device__ constexpr uint32_t umma_idesc_bf16(int M, int N) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+// instruction descriptor of kind::f16: D FP32, A and B BF16, N and M of the
+// instruction; a_mn / b_mn: the operand has M / N contiguous
+__host__ __device__ constexpr uint32_t umma_idesc_bf16(int M, int N, bool a_mn, bool b_mn) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((a_mn ? 1u : 0u) << 15) | ((b_mn ? 1u : 0u) << 16) |
+         ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t phase) {
+__device__ __forceinline__ void mbar_init(uint64_t* b) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(b)) : "memory");
+}
+// false when the wait ran out, or (give_up) another of the block has
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t phase, volatile int* failed, bool give_up = true) {
   const uint32_t a = smem_u32(bar);
-  for (long long i = 0; i < kTcSpin; i++) {
+  for (int i = 0; i < kTcSpin; i++) {
     uint32_t done;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
@@ -96,63 +116,36 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t phase) {
         : "r"(a), "r"(phase)
         : "memory");
     if (done) return true;
+    if (give_up && *failed) return false;
   }
   return false;
 }
-
-// 8 consecutive BF16 operands as one 16-byte load, zeros outside the matrix.
-// Channel counts are multiples of 8, so a run of 8 along the contiguous index
-// never crosses a tap or a row, and every run starts on a 16-byte boundary.
-__device__ __forceinline__ uint4 ld8(const __nv_bfloat16* p) { return *reinterpret_cast<const uint4*>(p); }
-__device__ __forceinline__ uint4 zero8() { return make_uint4(0u, 0u, 0u, 0u); }
-
-// A(m, k..k+7) where k is contiguous (forward: W[m][k])
-__device__ __forceinline__ uint4 a_k8(const ConvGemm& p, int m, int k) {
-  return (m < p.M && k < p.K) ? ld8(p.W + (size_t)m * p.K + k) : zero8();
-}
-// A(m..m+7, k) where m is contiguous (backward data: W[co][tap][m];
-// backward weights: dP[k][m])
-__device__ __forceinline__ uint4 a_m8(const ConvGemm& p, int m, int k) {
-  if (m >= p.M || k >= p.K) return zero8();
-  if (p.mode == G_BWD_DATA) {
-    const int tap = k / p.Cout, co = k - tap * p.Cout;
-    return ld8(p.W + ((size_t)co * kTaps + tap) * p.Cin + m);
-  }
-  return ld8(p.dP + (size_t)k * p.Cout + m);
-}
-// B(n, k..k+7) where k is contiguous (forward: X rows; backward data: dP rows)
-__device__ __forceinline__ uint4 b_k8(const ConvGemm& p, int n, int k) {
-  if (n >= p.N || k >= p.K) return zero8();
-  const int b = n / p.Z, z = n - b * p.Z;
-  if (p.mode == G_FWD) {
-    const int tap = k / p.Cin, ci = k - tap * p.Cin, zz = z + tap - kPad;
-    return (zz < 0 || zz >= p.Z) ? zero8() : ld8(p.X + ((size_t)b * p.Z + zz) * p.Cin + ci);
-  }
-  const int tap = k / p.Cout, co = k - tap * p.Cout, zz = z - tap + kPad;
-  return (zz < 0 || zz >= p.Z) ? zero8() : ld8(p.dP + ((size_t)b * p.Z + zz) * p.Cout + co);
-}
-// B(n..n+7, k) where n is contiguous (backward weights: X rows at z + tap)
-__device__ __forceinline__ uint4 b_n8(const ConvGemm& p, int n, int k) {
-  if (n >= p.N || k >= p.K) return zero8();
-  const int tap = n / p.Cin, ci = n - tap * p.Cin, b = k / p.Z, z = k - b * p.Z, zz = z + tap - kPad;
-  return (zz < 0 || zz >= p.Z) ? zero8() : ld8(p.X + ((size_t)b * p.Z + zz) * p.Cin + ci);
+__device__ __forceinline__ void tma3(void* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
+          smem_u32(dst)),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
+      : "memory");
 }
 
-// element (r, c) of a [rows][TK = 64] tile in the 128-byte-swizzled layout
-__device__ __forceinline__ int tc_off(int r, int c) {
-  return ((r >> 3) << 9) + ((r & 7) << 6) + ((((c >> 3) ^ (r & 7))) << 3) + (c & 7);
-}
-
-__global__ void __launch_bounds__(kTcThreads) k_conv_gemm_tc(ConvGemm p, int* err) {
+// tile (tn, m0) of one GEMM
+template <int MODE>
+__device__ __forceinline__ void conv_tile(const CUtensorMap& mapA, const CUtensorMap& mapB, const ConvGemm& p,
+                                          const int tn, const int m0, int* err) {
   extern __shared__ __align__(128) unsigned char tsm[];
-  // the stages start on a 1024-byte boundary (the swizzle pattern's period)
-  __nv_bfloat16* stage0 = reinterpret_cast<__nv_bfloat16*>(tsm + ((1024 - (smem_u32(tsm) & 1023)) & 1023));
-  __shared__ __align__(8) uint64_t mbar[2];
+  unsigned char* stage0 = tsm + ((1024 - (smem_u32(tsm) & 1023)) & 1023);
+  __shared__ __align__(8) uint64_t full[kTcStages], empty[kTcStages], done;
   __shared__ uint32_t tmem_base;
-  __shared__ int failed;
+  __shared__ volatile int failed;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
-  const bool a_mfast = p.mode != G_FWD, b_nfast = p.mode == G_BWD_W;
+  constexpr int ns = kTcStages;
+  constexpr bool a_mn = MODE != G_FWD, b_mn = MODE == G_BWD_W;
+  // the tile's n: levels z0 .. of sample nb, or channels c0n .. of a tap
+  const int per = MODE == G_BWD_W ? (p.Cin + TN - 1) / TN : (p.Z + TN - 1) / TN;
+  const int nb = tn / per, n0 = (tn - nb * per) * TN;
+  // the K slices: (tap, 64 channels), or (sample, 64 levels)
+  const int ks = MODE == G_BWD_W ? (p.Z + TK - 1) / TK : ((MODE == G_FWD ? p.Cin : p.Cout) + TK - 1) / TK;
+  const int nk = (MODE == G_BWD_W ? p.B : kTaps) * ks;
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
                  "r"(TN));
@@ -160,96 +153,92 @@ __global__ void __launch_bounds__(kTcThreads) k_conv_gemm_tc(ConvGemm p, int* er
   }
   if (tid == 0) {
     failed = 0;
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&mbar[0])));
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&mbar[1])));
-    asm volatile("fence.mbarrier_init.release.cluster;");
+    for (int s = 0; s < ns; s++) {
+      mbar_init(&full[s]);
+      mbar_init(&empty[s]);
+    }
+    mbar_init(&done);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = tmem_base;
-  const int nk = (p.K + TK - 1) / TK;
-  uint32_t phase[2] = {0, 0};
-  constexpr uint32_t idesc = umma_idesc_bf16(TM, TN);
-  for (int kt = 0; kt < nk && !failed; kt++) {
-    const int s = kt & 1, k0 = kt * TK;
-    __nv_bfloat16* As = stage0 + (size_t)s * kTcStageElems;
-    __nv_bfloat16* Bs = As + TM * TK;
-    if (kt >= 2) {   // the MMAs of slice kt - 2 read this stage
-      if (!mbar_wait(&mbar[s], phase[s])) {
-        if (tid == 0) { failed = 1; atomicExch(err, 1); }
+  if (warp == 0) {
+    if (lane == 0) {
+      int kt = 0, s = 0, ph = 1;   // ph: the parity of the slot's last use
+      for (; kt < nk; kt++, s = s + 1 == ns ? 0 : s + 1, ph ^= s == 0) {
+        const int k1 = kt / ks, k0 = (kt - k1 * ks) * TK;
+        if (kt >= ns && !mbar_wait(&empty[s], ph, &failed)) {
+          failed = 1;
+          atomicExch(err, 1);
+          break;
+        }
+        unsigned char *A = stage0 + (size_t)s * kTcStageBytes, *Bt = A + kTcABytes;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&full[s])),
+                     "r"(kTcStageBytes)
+                     : "memory");
+        if (MODE == G_FWD) {
+          tma3(A, &mapA, k0, k1, m0, &full[s]);
+          tma3(Bt, &mapB, k0, n0 + k1 - kPad, nb, &full[s]);
+        } else if (MODE == G_BWD_DATA) {
+          tma3(A, &mapA, m0, k1, k0, &full[s]);
+          tma3(A + kTcABytes / 2, &mapA, m0 + 64, k1, k0, &full[s]);
+          tma3(Bt, &mapB, k0, n0 - k1 + kPad, nb, &full[s]);
+        } else {
+          tma3(A, &mapA, m0, k0, k1, &full[s]);
+          tma3(A + kTcABytes / 2, &mapA, m0 + 64, k0, k1, &full[s]);
+          tma3(Bt, &mapB, n0, k0 + nb - kPad, k1, &full[s]);
+        }
       }
-      phase[s] ^= 1;
+      if (failed)   // the copies in flight
+        for (int i = kt > ns ? kt - ns : 0; i < kt; i++) mbar_wait(&full[i % ns], (i / ns) & 1, &failed, false);
     }
-    __syncthreads();
-    if (failed) break;
-    // one 16-byte load per thread and pass: a core-matrix row when K is the
-    // contiguous index, else 8 rows of one K column
-    // K contiguous: 8 threads load one row's 128 bytes and fill its line;
-    // M or N contiguous: a thread loads 8 rows of one K column, and the
-    // threads of a warp take consecutive columns (conflict-free stores)
-    if (!a_mfast) {
-      for (int i = tid; i < TM * (TK / 8); i += kTcThreads) {
-        const int r = i / (TK / 8), c = 8 * (i % (TK / 8));
-        *reinterpret_cast<uint4*>(&As[tc_off(r, c)]) = a_k8(p, m0 + r, k0 + c);
-      }
-    } else {
-      for (int i = tid; i < (TM / 8) * TK; i += kTcThreads) {
-        const int c = i % TK, r = 8 * (i / TK);
-        const uint4 v = a_m8(p, m0 + r, k0 + c);
-        const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&v);
+    __syncwarp();
+  } else if (warp == 1) {
+    if (lane == 0) {
+      constexpr uint32_t idesc = umma_idesc_bf16(TM, TN, a_mn, b_mn);
+      int s = 0, ph = 0;
+      for (int kt = 0; kt < nk; kt++, s = s + 1 == ns ? 0 : s + 1, ph ^= s == 0) {
+        if (!mbar_wait(&full[s], ph, &failed)) {
+          failed = 1;
+          atomicExch(err, 1);
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        const uint32_t a0 = smem_u32(stage0) + s * kTcStageBytes, b0 = a0 + kTcABytes;
 #pragma unroll
-        for (int j = 0; j < 8; j++) As[tc_off(r + j, c)] = e[j];
+        for (int kk = 0; kk < TK / 16; kk++) {
+          // K = 16 per instruction: 32 bytes of every row, or 16 rows of 128
+          const uint64_t da = umma_desc_sw128(a0 + (a_mn ? 2048 : 32) * kk, a_mn);
+          const uint64_t db = umma_desc_sw128(b0 + (b_mn ? 2048 : 32) * kk, b_mn);
+          const uint32_t acc = (kt > 0 || kk > 0) ? 1u : 0u;
+          asm volatile(
+              "{\n\t.reg .pred p;\n\t"
+              "setp.ne.b32 p, %4, 0;\n\t"
+              "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+              ::"r"(tmem), "l"(da), "l"(db), "r"(idesc), "r"(acc));
+        }
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                         smem_u32(kt + 1 < nk ? &empty[s] : &done))
+                     : "memory");   // the last covers every instruction before it
       }
     }
-    if (!b_nfast) {
-      for (int i = tid; i < TN * (TK / 8); i += kTcThreads) {
-        const int r = i / (TK / 8), c = 8 * (i % (TK / 8));
-        *reinterpret_cast<uint4*>(&Bs[tc_off(r, c)]) = b_k8(p, n0 + r, k0 + c);
-      }
-    } else {
-      for (int i = tid; i < (TN / 8) * TK; i += kTcThreads) {
-        const int c = i % TK, r = 8 * (i / TK);
-        const uint4 v = b_n8(p, n0 + r, k0 + c);
-        const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&v);
-#pragma unroll
-        for (int j = 0; j < 8; j++) Bs[tc_off(r + j, c)] = e[j];
-      }
-    }
-    // the generic-proxy stores must be visible to the tensor cores' async proxy
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncthreads();
-    if (tid == 0) {
-      asm volatile("tcgen05.fence::after_thread_sync;");
-      const uint32_t a0 = smem_u32(As), b0 = smem_u32(Bs);
-#pragma unroll
-      for (int kk = 0; kk < TK / 16; kk++) {
-        // K = 16 per instruction: bytes 32 kk .. 32 kk + 31 of every row
-        const uint64_t da = umma_desc_sw128(a0 + 32 * kk);
-        const uint64_t db = umma_desc_sw128(b0 + 32 * kk);
-        const uint32_t acc = (kt > 0 || kk > 0) ? 1u : 0u;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "setp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-            ::"r"(tmem), "l"(da), "l"(db), "r"(idesc), "r"(acc));
-      }
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                       smem_u32(&mbar[s]))
-                   : "memory");
-    }
+    __syncwarp();
   }
-  // the last commit covers every MMA issued before it
-  if (!failed && nk > 0) {
-    const int s = (nk - 1) & 1;
-    if (!mbar_wait(&mbar[s], phase[s]) && tid == 0) { failed = 1; atomicExch(err, 1); }
+  const bool ok = mbar_wait(&done, 0, &failed);
+  if (!ok && !failed) {
+    failed = 1;
+    atomicExch(err, 1);
   }
-  __syncthreads();
+  __syncwarp();
   asm volatile("tcgen05.fence::after_thread_sync;");
-  if (!failed) {
+  if (__all_sync(0xffffffffu, ok)) {
     // warp w reads tensor-memory lanes 32w..32w+31: row m0 + 32w + lane
     const int m = m0 + 32 * warp + lane;
+    const int nend = (MODE == G_BWD_W ? p.Cin : p.Z) - n0;   // columns of the tile inside C
     for (int c = 0; c < TN; c += 8) {
+      if (c >= nend) break;
       uint32_t v[8];
       asm volatile(
           "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -257,23 +246,33 @@ __global__ void __launch_bounds__(kTcThreads) k_conv_gemm_tc(ConvGemm p, int* er
           : "r"(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)c));
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
       if (m >= p.M) continue;
+      if (MODE == G_BWD_W) {   // channel counts are multiples of 8: 8 whole columns, 32-byte aligned
+        float4* o = reinterpret_cast<float4*>(p.outF + ((size_t)m * kTaps + nb) * p.Cin + n0 + c);
+        o[0] = make_float4(__uint_as_float(v[0]), __uint_as_float(v[1]), __uint_as_float(v[2]), __uint_as_float(v[3]));
+        o[1] = make_float4(__uint_as_float(v[4]), __uint_as_float(v[5]), __uint_as_float(v[6]), __uint_as_float(v[7]));
+        continue;
+      }
+      const size_t o0 = ((size_t)nb * p.Z + n0 + c) * p.M + m;
+      if (MODE == G_FWD) {
+        const float bias = p.bias[m];
 #pragma unroll
-      for (int e = 0; e < 8; e++) {
-        const int n = n0 + c + e;
-        if (n >= p.N) break;
-        float x = __uint_as_float(v[e]);
-        if (p.mode == G_FWD) {
-          x += p.bias[m];
-          const size_t o = (size_t)n * p.M + m;
+        for (int e = 0; e < 8; e++) {
+          if (c + e >= nend) break;
+          const float x = __uint_as_float(v[e]) + bias;
+          const size_t o = o0 + (size_t)e * p.M;
           if (p.outF) p.outF[o] = x;
           if (p.outB) p.outB[o] = __float2bfloat16(p.relu ? fmaxf(x, 0.f) : x);
-        } else if (p.mode == G_BWD_DATA) {
-          const size_t o = (size_t)n * p.M + m;
-          if (p.mask && !(__bfloat162float(p.mask[o]) > 0.f)) x = 0.f;
-          if (p.outF) p.outF[o] = x;
-          if (p.outB) p.outB[o] = __float2bfloat16(x);
-        } else {
-          p.outF[(size_t)m * p.N + n] = x;
+        }
+      } else {
+        __nv_bfloat16 k[8];
+#pragma unroll
+        for (int e = 0; e < 8; e++)
+          if (c + e < nend) k[e] = p.mask[o0 + (size_t)e * p.M];
+#pragma unroll
+        for (int e = 0; e < 8; e++) {
+          if (c + e >= nend) break;
+          const float x = __bfloat162float(k[e]) > 0.f ? __uint_as_float(v[e]) : 0.f;
+          p.outB[o0 + (size_t)e * p.M] = __float2bfloat16(x);
         }
       }
     }
@@ -281,6 +280,29 @@ __global__ void __launch_bounds__(kTcThreads) k_conv_gemm_tc(ConvGemm p, int* er
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TN));
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(kTcThreads) k_conv_gemm_tc(const __grid_constant__ CUtensorMap mapA,
+                                                              const __grid_constant__ CUtensorMap mapB,
+                                                              const __grid_constant__ ConvGemm p, int* err) {
+  conv_tile<MODE>(mapA, mapB, p, blockIdx.x, blockIdx.y * TM, err);
+}
+
+// the weight gradients of every layer in one launch, once the last dP is
+// known: a layer alone has 40 to 160 tiles, each a chain of B * Z / 64 slices
+// (four launches of 23 to 28 us at 13 samples of 256 levels; together 48 us)
+struct DwLayers {
+  CUtensorMap dp[kMaxLayers], x[kMaxLayers];
+  ConvGemm g[kMaxLayers];
+  int first[kMaxLayers + 1];   // first block of each layer
+};
+__global__ void __launch_bounds__(kTcThreads) k_conv_gemm_tc_dw(const __grid_constant__ DwLayers d, int* err) {
+  int l = 0;
+  while ((int)blockIdx.x >= d.first[l + 1]) l++;
+  const ConvGemm& p = d.g[l];
+  const int t = blockIdx.x - d.first[l], nt = kTaps * ((p.Cin + TN - 1) / TN);
+  conv_tile<G_BWD_W>(d.dp[l], d.x[l], p, t % nt, (t / nt) * TM, err);
 }
 
 __global__ void k_to_bf16(const float* __restrict__ x, __nv_bfloat16* __restrict__ y, size_t n) {
@@ -309,13 +331,41 @@ __global__ void k_mse(const float* __restrict__ out, const float* __restrict__ t
   }
 }
 
-// dbias[co] = sum over (b,z) of dP[b][z][co]
-__global__ void k_bias_grad(const __nv_bfloat16* __restrict__ dP, int rows, int C, float* __restrict__ db) {
-  const int co = blockIdx.x * blockDim.x + threadIdx.x;
-  if (co >= C) return;
-  float s = 0.f;
-  for (int r = 0; r < rows; r++) s += __bfloat162float(dP[(size_t)r * C + co]);
-  db[co] = s;
+// dbias[co] = sum over (b,z) of dP[b][z][co], every layer in one launch. A
+// block takes 16 channels: two threads read a row's 32 bytes, 128 rows at a
+// time, and the block's partial sums are added as a tree (one thread per
+// channel over all rows was one chain of dependent additions: 765 us for 3328
+// rows and four layers; now 19).
+constexpr int kBiasThreads = 256;
+struct BiasLayers {
+  const __nv_bfloat16* dP[kMaxLayers];
+  float* db[kMaxLayers];
+  int C[kMaxLayers];
+};
+__global__ void __launch_bounds__(kBiasThreads) k_bias_grad(const __grid_constant__ BiasLayers a, int rows) {
+  const int C = a.C[blockIdx.y];
+  if (16 * (int)blockIdx.x >= C) return;
+  const __nv_bfloat16* __restrict__ dP = a.dP[blockIdx.y];
+  float* __restrict__ db = a.db[blockIdx.y];
+  __shared__ float red[kBiasThreads / 2][17];
+  const int half = threadIdx.x & 1, r0 = threadIdx.x >> 1, c = 16 * blockIdx.x + 8 * half;
+  float s[8] = {};
+  if (c < C)   // channel counts are multiples of 8
+#pragma unroll 4
+    for (int r = r0; r < rows; r += kBiasThreads / 2) {
+      const uint4 v = *reinterpret_cast<const uint4*>(dP + (size_t)r * C + c);
+      const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&v);
+#pragma unroll
+      for (int k = 0; k < 8; k++) s[k] += __bfloat162float(e[k]);
+    }
+#pragma unroll
+  for (int k = 0; k < 8; k++) red[r0][8 * half + k] = s[k];
+  __syncthreads();
+  for (int n = kBiasThreads / 4; n > 0; n >>= 1) {
+    for (int i = threadIdx.x; i < n * 16; i += kBiasThreads) red[i >> 4][i & 15] += red[(i >> 4) + n][i & 15];
+    __syncthreads();
+  }
+  if (threadIdx.x < 16 && 16 * (int)blockIdx.x + (int)threadIdx.x < C) db[16 * blockIdx.x + threadIdx.x] = red[0][threadIdx.x];
 }
 
 // Adam (Kingma & Ba 2015) on the FP32 master weights; refreshes the BF16
@@ -356,6 +406,12 @@ struct sf_net {
   long long t = 0;                   // Adam steps taken
   cudaStream_t st = nullptr;
   int* err = nullptr;                // set by a GEMM block whose bounded wait ran out
+  // tensor maps of each layer: W in boxes of 128 and of 64 output channels,
+  // the layer's input and the gradient of its pre-activation
+  struct Maps {
+    CUtensorMap wf, wb, x, dp;
+  };
+  std::vector<Maps> maps;
 };
 
 namespace {
@@ -371,14 +427,31 @@ int nfail(int code, const std::string& m) {
     if (e_ != cudaSuccess) return nfail(SF_ECUDA, std::string(#x) + ": " + cudaGetErrorString(e_)); \
   } while (0)
 
-int gemm(sf_net* n, ConvGemm p) {
-  switch (p.mode) {
-    case G_FWD: p.M = p.Cout; p.N = p.B * p.Z; p.K = kTaps * p.Cin; break;
-    case G_BWD_DATA: p.M = p.Cin; p.N = p.B * p.Z; p.K = kTaps * p.Cout; break;
-    default: p.M = p.Cout; p.N = kTaps * p.Cin; p.K = p.B * p.Z; break;
-  }
-  dim3 grid((p.N + TN - 1) / TN, (p.M + TM - 1) / TM);
-  k_conv_gemm_tc<<<grid, kTcThreads, kTcSmem, n->st>>>(p, n->err);
+// a BF16 tensor [d2][d1][d0] in boxes of 64 x b1 x b2 with the 128-byte swizzle
+int conv_map(CUtensorMap* m, const __nv_bfloat16* base, int d0, int d1, int d2, int b1, int b2) {
+  void* fn = nullptr;
+  cudaDriverEntryPointQueryResult q;
+  if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) != cudaSuccess ||
+      q != cudaDriverEntryPointSuccess || !fn)
+    return -1;
+  const cuuint64_t dims[3] = {(cuuint64_t)d0, (cuuint64_t)d1, (cuuint64_t)d2};
+  const cuuint64_t strides[2] = {(cuuint64_t)d0 * 2, (cuuint64_t)d0 * d1 * 2};
+  const cuuint32_t box[3] = {64, (cuuint32_t)b1, (cuuint32_t)b2}, es[3] = {1, 1, 1};
+  const CUresult r = reinterpret_cast<PFN_cuTensorMapEncodeTiled>(fn)(
+      m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<__nv_bfloat16*>(base), dims, strides, box, es,
+      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : -1;
+}
+
+unsigned tiles(int a, int b) { return (unsigned)((a + b - 1) / b); }
+
+int gemm(sf_net* n, int l, GemmMode mode, ConvGemm p) {
+  const sf_net::Maps& t = n->maps[l];
+  p.M = mode == G_FWD ? p.Cout : p.Cin;
+  const dim3 grid(p.B * tiles(p.Z, TN), tiles(p.M, TM));
+  if (mode == G_FWD) k_conv_gemm_tc<G_FWD><<<grid, kTcThreads, kTcSmem, n->st>>>(t.wf, t.x, p, n->err);
+  else k_conv_gemm_tc<G_BWD_DATA><<<grid, kTcThreads, kTcSmem, n->st>>>(t.wb, t.dp, p, n->err);
   NCK(cudaGetLastError());
   return SF_OK;
 }
@@ -386,16 +459,13 @@ int gemm(sf_net* n, ConvGemm p) {
 int forward(sf_net* n, int B, bool keep_out) {
   for (int l = 0; l < n->nl; l++) {
     ConvGemm p{};
-    p.mode = G_FWD;
     p.B = B; p.Z = n->Z; p.Cin = n->ch[l]; p.Cout = n->ch[l + 1];
-    p.W = n->wb + n->woff[l];
-    p.X = n->act[l];
     p.bias = n->w + n->boff[l];
     const bool last = l == n->nl - 1;
     p.outF = last ? n->out : nullptr;
     p.outB = last ? nullptr : n->act[l + 1];
     p.relu = last ? 0 : 1;
-    int rc = gemm(n, p);
+    int rc = gemm(n, l, G_FWD, p);
     if (rc) return rc;
   }
   (void)keep_out;
@@ -406,28 +476,34 @@ int forward(sf_net* n, int B, bool keep_out) {
 int backward(sf_net* n, int B) {
   const size_t nout = (size_t)B * n->Z * n->ch[n->nl];
   NCK(cudaMemsetAsync(n->loss, 0, sizeof(double), n->st));
-  k_mse<<<blocks_for(nout, 256), 256, 0, n->st>>>(n->out, n->tgt, n->dP[n->nl - 1], nout, n->loss);
-  for (int l = n->nl - 1; l >= 0; l--) {
+  k_mse<<<std::min(blocks_for(nout, 256), 592u), 256, 0, n->st>>>(n->out, n->tgt, n->dP[n->nl - 1], nout, n->loss);
+  for (int l = n->nl - 1; l > 0; l--) {   // dP of layer l-1 = (W^T * dP_l) where its ReLU was active
     ConvGemm p{};
     p.B = B; p.Z = n->Z; p.Cin = n->ch[l]; p.Cout = n->ch[l + 1];
-    p.W = n->wb + n->woff[l];
-    p.X = n->act[l];
-    p.dP = n->dP[l];
-    p.mode = G_BWD_W;
-    p.outF = n->gr + n->woff[l];
-    int rc = gemm(n, p);
+    p.outB = n->dP[l - 1];
+    p.mask = n->act[l];
+    int rc = gemm(n, l, G_BWD_DATA, p);
     if (rc) return rc;
-    k_bias_grad<<<(p.Cout + 127) / 128, 128, 0, n->st>>>(n->dP[l], B * n->Z, p.Cout, n->gr + n->boff[l]);
-    if (l > 0) {   // dP of layer l-1 = (W^T * dP_l) where its ReLU was active
-      ConvGemm q = p;
-      q.mode = G_BWD_DATA;
-      q.outF = nullptr;
-      q.outB = n->dP[l - 1];
-      q.mask = n->act[l];
-      rc = gemm(n, q);
-      if (rc) return rc;
-    }
   }
+  DwLayers d;
+  BiasLayers bl;
+  int blocks = 0, cmax = 0;
+  for (int l = 0; l < n->nl; l++) {
+    ConvGemm& p = d.g[l] = ConvGemm{};
+    p.B = B; p.Z = n->Z; p.Cin = n->ch[l]; p.M = p.Cout = n->ch[l + 1];
+    p.outF = n->gr + n->woff[l];
+    d.dp[l] = n->maps[l].dp;
+    d.x[l] = n->maps[l].x;
+    d.first[l] = blocks;
+    blocks += (int)(kTaps * tiles(p.Cin, TN) * tiles(p.M, TM));
+    bl.dP[l] = n->dP[l];
+    bl.db[l] = n->gr + n->boff[l];
+    bl.C[l] = p.Cout;
+    cmax = std::max(cmax, p.Cout);
+  }
+  d.first[n->nl] = blocks;
+  k_conv_gemm_tc_dw<<<blocks, kTcThreads, kTcSmem, n->st>>>(d, n->err);
+  k_bias_grad<<<dim3(tiles(cmax, 16), n->nl), kBiasThreads, 0, n->st>>>(bl, B * n->Z);
   NCK(cudaGetLastError());
   return SF_OK;
 }
@@ -463,7 +539,7 @@ static int net_status(sf_net* n) {
 
 int sf_net_create(int nlayers, const int* channels, int Z, int max_batch, unsigned long long seed, void* stream,
                   sf_net** out) {
-  if (!out || nlayers < 1 || nlayers > 16 || !channels || Z < 1 || max_batch < 1)
+  if (!out || nlayers < 1 || nlayers > kMaxLayers || !channels || Z < 1 || max_batch < 1)
     return nfail(SF_EINVAL, "bad argument");
   for (int l = 0; l <= nlayers; l++)
     if (channels[l] < 1 || channels[l] % 8) return nfail(SF_EINVAL, "channel counts must be positive multiples of 8");
@@ -509,8 +585,20 @@ int sf_net_create(int nlayers, const int* channels, int Z, int max_batch, unsign
   if (cudaMalloc(&n->xin, sizeof(float) * rows * n->ch[0]) != cudaSuccess) return bail("cudaMalloc input");
   if (cudaMalloc(&n->loss, sizeof(double)) != cudaSuccess) return bail("cudaMalloc loss");
   if (cudaMalloc(&n->err, sizeof(int)) != cudaSuccess) return bail("cudaMalloc status");
-  if (cudaMemset(n->err, 0, sizeof(int)) != cudaSuccess ||
-      cudaFuncSetAttribute(k_conv_gemm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem) != cudaSuccess) {
+  bool set = cudaMemset(n->err, 0, sizeof(int)) == cudaSuccess;
+  const int lim = (int)kTcSmem;
+  for (auto* k : {k_conv_gemm_tc<G_FWD>, k_conv_gemm_tc<G_BWD_DATA>})
+    set = set && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) == cudaSuccess;
+  set = set && cudaFuncSetAttribute(k_conv_gemm_tc_dw, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) == cudaSuccess;
+  n->maps.resize(nlayers);
+  for (int l = 0; l < nlayers && set; l++) {
+    const int ci = n->ch[l], co = n->ch[l + 1];
+    sf_net::Maps& t = n->maps[l];
+    const __nv_bfloat16* W = n->wb + n->woff[l];
+    set = conv_map(&t.wf, W, ci, kTaps, co, 1, TM) == 0 && conv_map(&t.wb, W, ci, kTaps, co, 1, TK) == 0 &&
+          conv_map(&t.x, n->act[l], ci, Z, max_batch, TN, 1) == 0 && conv_map(&t.dp, n->dP[l], co, Z, max_batch, TN, 1) == 0;
+  }
+  if (!set) {
     sf_net_destroy(n);
     return nfail(SF_ECUDA, "setting up the tensor-core GEMM");
   }
