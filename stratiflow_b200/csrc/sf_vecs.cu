@@ -28,7 +28,7 @@ struct sf_vecs {
   float2* d = nullptr;      // [nvec][5][N3][Pp]
   double* red = nullptr;    // reduction scratch
   int cap_red = 0;
-  double* coef = nullptr;   // block-update coefficients
+  float* coef = nullptr;    // block-update coefficients
   size_t cap_coef = 0;
   const float* zc = nullptr;
   cudaStream_t st = nullptr;
@@ -97,94 +97,205 @@ __global__ void k_dots(Geo g, const float2* __restrict__ base, size_t stride, co
   }
 }
 
-// Block Gram matrix: part[c][i][k] = the share of level chunk c (kGramLevels
-// levels of one field) of Dot(V_i, W_k), i < nv, k < nw <= kMaxBlock. One
-// warp per (chunk, field, i): lanes stride over the modes and keep one FP64
-// sum per k; the partial sums are added in a fixed order afterwards.
+// Block Gram matrix: part[c][i][k] = the share of chunk c (kGramLevels levels
+// of one field) of Dot(V_i, W_k), i < nv, k < nw <= kMaxBlock, FP64.
+//
+// A contraction over the modes and levels, on the FP64 tensor instruction
+// (m8n8k4): a warp keeps MA x NA tiles of 8 x 8 sums. The order of the k
+// within a sum is free, so a lane loads four consecutive floats of its row of
+// V (and of W) with one 16-byte load and feeds one of them to each of four
+// instructions; nothing goes through shared memory. The four warps of a block
+// take the levels of its chunk in turn and add their sums at the end. Bound
+// by the FP64 rate (1.3 GFLOP for 320 x 16 vectors of 256x1x256, 37 us) and
+// the one reading of V (29 us); with one dot product per lane and pair, each
+// converting its two floats and reading W through the L1, 413 us; now 64.
 constexpr int kGramLevels = 8;
 constexpr int kMaxBlock = 32;
 
-template <int NW>
-__global__ void __launch_bounds__(256) k_gram(Geo g, const float2* __restrict__ V, int nv,
+__device__ __forceinline__ void mma_f64(double (&c)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+               : "+d"(c[0]), "+d"(c[1])
+               : "d"(a), "d"(b));
+}
+
+template <int MA, int NA>
+__global__ void __launch_bounds__(128) k_gram(Geo g, const float2* __restrict__ V, int nv,
                                                const float2* __restrict__ W, int nw, size_t stride,
                                                const float* __restrict__ zc, double Ri, double* __restrict__ part) {
-  const int chunk = blockIdx.x, f = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int i = blockIdx.z * 8 + warp;
-  if (i >= nv) return;
-  const int nch = gridDim.x;
-  double acc[NW];
+  const int nch = (g.N3 + kGramLevels - 1) / kGramLevels;
+  const int fi = blockIdx.x / nch, chunk = blockIdx.x - fi * nch;
+  const int f = g.dim3 || fi == 0 ? fi : fi + 1;   // 2D: u1, u3, b
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = lane >> 2, q = lane & 3;
+  const int i0 = blockIdx.y * 8 * MA;
+  double acc[MA][NA][2] = {};
+  const int steps = (2 * g.P + 15) / 16;   // of 16 floats of a level's row
+  for (int j = chunk * kGramLevels + warp; j < min(g.N3, (chunk + 1) * kGramLevels); j += 4) {
+    const double wz = (double)zc[(f == 2 ? ZC_WZD : ZC_WZN) * g.N3 + j] * (f == 3 ? Ri : 1.0);
+    if (wz == 0.0) continue;
+    const size_t row = ((size_t)f * g.N3 + j) * g.Pp;
+    // rows past the end repeat the last one: their sums are not written
+    const float4 *av[MA], *bv[NA];
 #pragma unroll
-  for (int k = 0; k < NW; k++) acc[k] = 0.0;
-  if (f != 1 || g.dim3) {
-    for (int j = chunk * kGramLevels; j < min(g.N3, (chunk + 1) * kGramLevels); j++) {
-      const double wz = (double)zc[(f == 2 ? ZC_WZD : ZC_WZN) * g.N3 + j] * (f == 3 ? Ri : 1.0);
-      if (wz == 0.0) continue;
-      const size_t row = ((size_t)f * g.N3 + j) * g.Pp;
-      const float2* v = V + (size_t)i * stride + row;
-      for (int m = lane; m < g.P; m += 32) {
-        const float2 a = v[m];
-        const double wm = (m == 0) ? wz : 2.0 * wz;
+    for (int t = 0; t < MA; t++)
+      av[t] = reinterpret_cast<const float4*>(V + (size_t)min(i0 + 8 * t + r, nv - 1) * stride + row) + q;
 #pragma unroll
-        for (int k = 0; k < NW; k++) {
-          if (k < nw) {
-            const float2 b = W[(size_t)k * stride + row + m];
-            acc[k] += wm * ((double)a.x * b.x + (double)a.y * b.y);
-          }
+    for (int t = 0; t < NA; t++)
+      bv[t] = reinterpret_cast<const float4*>(W + (size_t)min(8 * t + r, nw - 1) * stride + row) + q;
+    // the loads of the next step go ahead of this step's arithmetic
+    float4 na[MA], nb[NA];
+#pragma unroll
+    for (int t = 0; t < MA; t++) na[t] = av[t][0];
+#pragma unroll
+    for (int t = 0; t < NA; t++) nb[t] = bv[t][0];
+    for (int s = 0; s < steps; s++) {
+      float a[MA][4], b[NA][4];
+      const int left = 2 * g.P - (16 * s + 4 * q);   // floats of kept modes from this lane's on
+#pragma unroll
+      for (int t = 0; t < MA; t++) {
+        const float4 x = na[t];
+        a[t][0] = left > 0 ? x.x : 0.f;
+        a[t][1] = left > 1 ? x.y : 0.f;
+        a[t][2] = left > 2 ? x.z : 0.f;
+        a[t][3] = left > 3 ? x.w : 0.f;
+      }
+#pragma unroll
+      for (int t = 0; t < NA; t++) {
+        const float4 x = nb[t];
+        b[t][0] = left > 0 ? x.x : 0.f;
+        b[t][1] = left > 1 ? x.y : 0.f;
+        b[t][2] = left > 2 ? x.z : 0.f;
+        b[t][3] = left > 3 ? x.w : 0.f;
+      }
+      const int n = min(s + 1, steps - 1);
+#pragma unroll
+      for (int t = 0; t < MA; t++) na[t] = av[t][4 * n];
+#pragma unroll
+      for (int t = 0; t < NA; t++) nb[t] = bv[t][4 * n];
+#pragma unroll
+      for (int e = 0; e < 4; e++) {
+        // the (0,0) mode counts once, the others twice (Integration.h:282-311)
+        const double w = (s == 0 && q == 0 && e < 2) ? wz : 2.0 * wz;
+        double bd[NA];
+#pragma unroll
+        for (int t = 0; t < NA; t++) bd[t] = w * (double)b[t][e];
+#pragma unroll
+        for (int u = 0; u < MA; u++) {
+          const double ad = (double)a[u][e];
+#pragma unroll
+          for (int t = 0; t < NA; t++) mma_f64(acc[u][t], ad, bd[t]);
         }
       }
     }
   }
+  // the warps' sums: element (row r, columns 2q, 2q + 1) of each 8 x 8 tile
+  __shared__ double sum[3][MA * NA * 2][32];
+  if (warp > 0) {
 #pragma unroll
-  for (int k = 0; k < NW; k++) {
-    double t = acc[k];
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    acc[k] = t;
-  }
-  if (lane == 0) {
-    double* out = part + (((size_t)f * nch + chunk) * nv + i) * nw;
+    for (int u = 0; u < MA; u++)
 #pragma unroll
-    for (int k = 0; k < NW; k++)
-      if (k < nw) out[k] = acc[k];
+      for (int t = 0; t < NA; t++)
+#pragma unroll
+        for (int e = 0; e < 2; e++) sum[warp - 1][(u * NA + t) * 2 + e][lane] = acc[u][t][e];
   }
+  __syncthreads();
+  if (warp > 0) return;
+#pragma unroll
+  for (int u = 0; u < MA; u++)
+#pragma unroll
+    for (int t = 0; t < NA; t++)
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const int k = (u * NA + t) * 2 + e, i = i0 + 8 * u + r, c = 8 * t + 2 * q + e;
+        if (i < nv && c < nw)
+          part[((size_t)blockIdx.x * nv + i) * nw + c] = acc[u][t][e] + sum[0][k][lane] + sum[1][k][lane] + sum[2][k][lane];
+      }
 }
 
-// out[i][k] = sum over the 4 * nch partials, in order
-__global__ void k_gram_sum(const double* __restrict__ part, int nparts, int nvw, double* __restrict__ out) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= nvw) return;
+// out[e] = the sum over the partials, in a fixed order: a block takes 32
+// entries, eight threads each
+__global__ void __launch_bounds__(256) k_gram_sum(const double* __restrict__ part, int nparts, int nvw,
+                                                  double* __restrict__ out) {
+  __shared__ double red[8][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, e = blockIdx.x * 32 + lane;
   double s = 0.0;
-  for (int c = 0; c < nparts; c++) s += part[(size_t)c * nvw + e];
+  if (e < nvw)
+    for (int c = w; c < nparts; c += 8) s += part[(size_t)c * nvw + e];
+  red[w][lane] = s;
+  __syncthreads();
+  if (w > 0 || e >= nvw) return;
+  for (int k = 1; k < 8; k++) s += red[k][lane];
   out[e] = s;
 }
 
-// W_k += alpha sum_i coef[i][k] V_i over u1,u2,u3,b, k < nw <= kMaxBlock
+// W_k += sum_i coef[i][k] V_i over u1,u2,u3,b, k < nw <= NW; coef holds NW
+// floats per i (alpha included, zeros past nw). Each warp of a block sums
+// every eighth V_i of the same 64 values of all NW results, two values per
+// lane, the results in packed pairs of k; the warps' sums are added in shared
+// memory. Bound by the one reading of V (320 vectors of 256x1x256: 252 MB, 39
+// us) and the FMAs (28 us); with the coefficients converted from FP64 by
+// every thread 347 us, now 98.
 template <int NW>
-__global__ void k_update(Geo g, float2* __restrict__ W, int nw, const float2* __restrict__ V, int nv, size_t stride,
-                         const double* __restrict__ coef, double alpha) {
-  const size_t n = (size_t)4 * g.fblk;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-    float2 acc[NW];
+__global__ void __launch_bounds__(256) k_update(Geo g, float2* __restrict__ W, int nw, const float2* __restrict__ V,
+                                                int nv, size_t stride, const float* __restrict__ coef) {
+  __shared__ float4 red[4][NW][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const size_t n = (size_t)4 * g.fblk;                      // a multiple of 64: Pp is one of 16, N3 of 4
+  const size_t e = (size_t)blockIdx.x * 64 + 2 * lane;      // this lane's two values
+  constexpr int H = (NW + 1) / 2;
+  float2 acc[4][H];   // re, im, re, im; (k, k + 1)
 #pragma unroll
-    for (int k = 0; k < NW; k++) acc[k] = make_float2(0.f, 0.f);
-    for (int i = 0; i < nv; i++) {
-      const float2 v = V[(size_t)i * stride + e];
-      const double* c = coef + (size_t)i * nw;
+  for (int c = 0; c < 4; c++)
 #pragma unroll
-      for (int k = 0; k < NW; k++) {
-        if (k < nw) {
-          const float ck = (float)(alpha * c[k]);
-          acc[k].x += ck * v.x;
-          acc[k].y += ck * v.y;
+    for (int h = 0; h < H; h++) acc[c][h] = make_float2(0.f, 0.f);
+  if (e < n) {
+#pragma unroll 4
+    for (int i = warp; i < nv; i += 8) {
+      const float4 v = *reinterpret_cast<const float4*>(V + (size_t)i * stride + e);
+      float2 c[H];
+      if (NW == 1) {
+        c[0] = make_float2(coef[i], 0.f);
+      } else {
+#pragma unroll
+        for (int h = 0; h < H; h += 2) {
+          const float4 x = __ldg(reinterpret_cast<const float4*>(coef + (size_t)i * NW) + h / 2);
+          c[h] = make_float2(x.x, x.y);
+          c[h + 1 < H ? h + 1 : h] = make_float2(x.z, x.w);
         }
       }
-    }
 #pragma unroll
-    for (int k = 0; k < NW; k++) {
-      if (k < nw) {
-        float2& w = W[(size_t)k * stride + e];
-        w = make_float2(w.x + acc[k].x, w.y + acc[k].y);
+      for (int h = 0; h < H; h++) {
+        acc[0][h] = __ffma2_rn(c[h], make_float2(v.x, v.x), acc[0][h]);
+        acc[1][h] = __ffma2_rn(c[h], make_float2(v.y, v.y), acc[1][h]);
+        acc[2][h] = __ffma2_rn(c[h], make_float2(v.z, v.z), acc[2][h]);
+        acc[3][h] = __ffma2_rn(c[h], make_float2(v.w, v.w), acc[3][h]);
       }
     }
+  }
+  // the upper four warps' sums to the lower four, then those to the results
+  for (int half = 1; half >= 0; half--) {
+    if ((warp >> 2) == half) {
+#pragma unroll
+      for (int k = 0; k < NW; k++) {
+        float4& r = red[warp & 3][k][lane];
+        const int h = k / 2;
+        const float4 x = k % 2 == 0 ? make_float4(acc[0][h].x, acc[1][h].x, acc[2][h].x, acc[3][h].x)
+                                    : make_float4(acc[0][h].y, acc[1][h].y, acc[2][h].y, acc[3][h].y);
+        r = half ? x : make_float4(r.x + x.x, r.y + x.y, r.z + x.z, r.w + x.w);
+      }
+    }
+    __syncthreads();
+  }
+  if (e >= n) return;
+  for (int k = warp; k < nw; k += 8) {
+    float4 s = red[0][k][lane];
+#pragma unroll
+    for (int w = 1; w < 4; w++) {
+      const float4 x = red[w][k][lane];
+      s = make_float4(s.x + x.x, s.y + x.y, s.z + x.z, s.w + x.w);
+    }
+    float4* w = reinterpret_cast<float4*>(W + (size_t)k * stride + e);
+    const float4 o = *w;
+    *w = make_float4(o.x + s.x, o.y + s.y, o.z + s.z, o.w + s.w);
   }
 }
 
@@ -452,21 +563,22 @@ int sf_vecs_gram(sf_vecs* v, int a, int na, sf_vecs* w, int b, int nb, double Ri
     return vfail(SF_EINVAL, "bad argument (1 <= nb <= 32)");
   const Geo& g = v->g;
   const int nch = (g.N3 + kGramLevels - 1) / kGramLevels;
-  const size_t nvw = (size_t)na * nb, parts = (size_t)4 * nch;
+  const size_t nvw = (size_t)na * nb, parts = (size_t)(g.dim3 ? 4 : 3) * nch;
   int rc = ensure_red(v, (int)(nvw * (parts + 1)));
   if (rc) return rc;
   double* part = v->red + nvw;
-  dim3 grid(nch, 4, (na + 7) / 8);
   auto* wd = w->d + (size_t)b * vstride(w->g);
   auto* vd = v->d + (size_t)a * vstride(g);
   const size_t vs = vstride(g);
-  if (nb <= 1) k_gram<1><<<grid, 256, 0, v->st>>>(g, vd, na, wd, nb, vs, v->zc, Ri, part);
-  else if (nb <= 4) k_gram<4><<<grid, 256, 0, v->st>>>(g, vd, na, wd, nb, vs, v->zc, Ri, part);
-  else if (nb <= 8) k_gram<8><<<grid, 256, 0, v->st>>>(g, vd, na, wd, nb, vs, v->zc, Ri, part);
-  else if (nb <= 16) k_gram<16><<<grid, 256, 0, v->st>>>(g, vd, na, wd, nb, vs, v->zc, Ri, part);
-  else k_gram<32><<<grid, 256, 0, v->st>>>(g, vd, na, wd, nb, vs, v->zc, Ri, part);
+  // 32 vectors of V per warp; 16 where there are no more, or where a block of 32 has twice the sums
+  auto launch = [&](auto* k, int ma) {
+    k<<<dim3((unsigned)parts, (na + 8 * ma - 1) / (8 * ma)), 128, 0, v->st>>>(g, vd, na, wd, nb, vs, v->zc, Ri, part);
+  };
+  if (nb <= 8) na <= 16 ? launch(k_gram<2, 1>, 2) : launch(k_gram<4, 1>, 4);
+  else if (nb <= 16) na <= 16 ? launch(k_gram<2, 2>, 2) : launch(k_gram<4, 2>, 4);
+  else launch(k_gram<2, 4>, 2);
   VCK(cudaGetLastError());
-  k_gram_sum<<<(unsigned)((nvw + 255) / 256), 256, 0, v->st>>>(part, (int)parts, (int)nvw, v->red);
+  k_gram_sum<<<(unsigned)((nvw + 31) / 32), 256, 0, v->st>>>(part, (int)parts, (int)nvw, v->red);
   VCK(cudaGetLastError());
   VCK(cudaMemcpyAsync(out, v->red, sizeof(double) * nvw, cudaMemcpyDeviceToHost, v->st));
   VCK(cudaStreamSynchronize(v->st));
@@ -480,27 +592,33 @@ int sf_vecs_update(sf_vecs* w, int b, int nb, double alpha, sf_vecs* v, int a, i
       b + nb > w->nvec)
     return vfail(SF_EINVAL, "bad argument (1 <= nb <= 32)");
   if (v == w && a < b + nb && b < a + na) return vfail(SF_EINVAL, "overlapping ranges");
-  const size_t nc = (size_t)na * nb;
-  if (nc > w->cap_coef) {
-    cudaFree(w->coef);
-    w->coef = nullptr;
-    w->cap_coef = 0;
-    VCK(cudaMalloc(&w->coef, sizeof(double) * nc));
-    w->cap_coef = nc;
+  // two launches above 16 vectors, whose sums would not fit the registers
+  for (int k0 = 0; k0 < nb; k0 += 16) {
+    const int k = std::min(16, nb - k0), NW = k <= 1 ? 1 : (k <= 4 ? 4 : (k <= 8 ? 8 : 16));
+    const size_t nc = (size_t)na * NW;
+    if (nc > w->cap_coef) {
+      cudaFree(w->coef);
+      w->coef = nullptr;
+      w->cap_coef = 0;
+      VCK(cudaMalloc(&w->coef, sizeof(float) * nc));
+      w->cap_coef = nc;
+    }
+    std::vector<float> c(nc, 0.f);
+    for (int i = 0; i < na; i++)
+      for (int j = 0; j < k; j++) c[(size_t)i * NW + j] = (float)(alpha * coef[(size_t)i * nb + k0 + j]);
+    // from pageable memory: c has been read when the call returns
+    VCK(cudaMemcpyAsync(w->coef, c.data(), sizeof(float) * nc, cudaMemcpyHostToDevice, w->st));
+    const Geo& g = w->g;
+    const unsigned blocks = (unsigned)(((size_t)4 * g.fblk + 63) / 64);
+    const size_t vs = vstride(g);
+    float2* wd = w->d + (size_t)(b + k0) * vs;
+    const float2* vd = v->d + (size_t)a * vs;
+    if (NW == 1) k_update<1><<<blocks, 256, 0, w->st>>>(g, wd, k, vd, na, vs, w->coef);
+    else if (NW == 4) k_update<4><<<blocks, 256, 0, w->st>>>(g, wd, k, vd, na, vs, w->coef);
+    else if (NW == 8) k_update<8><<<blocks, 256, 0, w->st>>>(g, wd, k, vd, na, vs, w->coef);
+    else k_update<16><<<blocks, 256, 0, w->st>>>(g, wd, k, vd, na, vs, w->coef);
+    VCK(cudaGetLastError());
   }
-  VCK(cudaMemcpyAsync(w->coef, coef, sizeof(double) * nc, cudaMemcpyHostToDevice, w->st));
-  const Geo& g = w->g;
-  const size_t n = (size_t)4 * g.fblk;
-  const unsigned blocks = (unsigned)std::min<size_t>((n + 255) / 256, 4096);
-  const size_t vs = vstride(g);
-  float2* wd = w->d + (size_t)b * vs;
-  const float2* vd = v->d + (size_t)a * vs;
-  if (nb <= 1) k_update<1><<<blocks, 256, 0, w->st>>>(g, wd, nb, vd, na, vs, w->coef, alpha);
-  else if (nb <= 4) k_update<4><<<blocks, 256, 0, w->st>>>(g, wd, nb, vd, na, vs, w->coef, alpha);
-  else if (nb <= 8) k_update<8><<<blocks, 256, 0, w->st>>>(g, wd, nb, vd, na, vs, w->coef, alpha);
-  else if (nb <= 16) k_update<16><<<blocks, 256, 0, w->st>>>(g, wd, nb, vd, na, vs, w->coef, alpha);
-  else k_update<32><<<blocks, 256, 0, w->st>>>(g, wd, nb, vd, na, vs, w->coef, alpha);
-  VCK(cudaGetLastError());
   return SF_OK;
 }
 
