@@ -380,6 +380,11 @@ int sf_net_gradient(sf_net* n, float* grad, double* loss);
  * (may be NULL) is the loss before step s */
 int sf_net_train(sf_net* n, int steps, double lr, double* losses);
 
+/* page-locked host memory (no counterpart in the reference), from which and
+ * to which copies run at the link's rate and without waiting */
+int sf_host_alloc(size_t bytes, void** ptr);
+int sf_host_free(void* ptr);
+
 /* waits for all work queued on the solver's stream */
 int sf_synchronize(sf_solver* s);
 

@@ -9,8 +9,11 @@ there is no CPU fallback: importing this package without it raises.
 """
 from __future__ import annotations
 
+import collections
 import ctypes as C
 import os
+import threading
+import weakref
 
 import numpy as np
 
@@ -35,7 +38,7 @@ EXPORTS = [
     "sf_vecs_dots", "sf_vecs_dot_sum", "sf_vecs_enforce_bcs", "sf_vecs_phase_shift", "sf_vecs_remove_average",
     "sf_vecs_zero_pressure", "sf_vecs_synchronize", "sf_set_tangent",
     "sf_net_create", "sf_net_destroy", "sf_net_num_params", "sf_net_get_params", "sf_net_set_params",
-    "sf_net_forward", "sf_net_set_data", "sf_net_gradient", "sf_net_train",
+    "sf_net_forward", "sf_net_set_data", "sf_net_gradient", "sf_net_train", "sf_host_alloc", "sf_host_free",
     "sf_vecs_gram", "sf_vecs_update", "sf_vecs_band", "sf_vecs_column", "sf_set_xpass_slabs", "sf_set_xy_bands", "sf_set_z_chunks", "sf_set_xpass_groups", "sf_set_xpass_kernel", "sf_set_z_kernel",
     "sf_ensemble_create", "sf_ensemble_destroy", "sf_ensemble_member", "sf_ensemble_step",
     "sf_ensemble_synchronize", "sf_ensemble_launch_count", "sf_ensemble_stream", "sf_ensemble_profile", "sf_set_base_device",
@@ -95,6 +98,7 @@ def load_library(path: str | None = None):
         "sf_net_num_params": [vp, C.POINTER(C.c_longlong)], "sf_net_get_params": [vp, fp],
         "sf_net_set_params": [vp, fp], "sf_net_forward": [vp, fp, i, fp], "sf_net_set_data": [vp, fp, fp, i],
         "sf_net_gradient": [vp, fp, dp], "sf_net_train": [vp, i, d, dp],
+        "sf_host_alloc": [C.c_size_t, C.POINTER(vp)], "sf_host_free": [vp],
         "sf_vecs_gram": [vp, i, i, vp, i, i, d, dp], "sf_vecs_update": [vp, i, i, d, vp, i, i, dp],
         "sf_vecs_band": [vp, i, i, i, i], "sf_vecs_column": [vp, i, i, i, fp, i], "sf_set_xpass_slabs": [vp, i], "sf_set_xy_bands": [vp, i], "sf_set_z_chunks": [vp, i], "sf_set_xpass_groups": [vp, i], "sf_set_xpass_kernel": [vp, i], "sf_set_z_kernel": [vp, i], "sf_set_base_device": [vp, i, vp],
         "sf_get_nodal": [vp, i, i, fp], "sf_set_nodal": [vp, i, i, fp], "sf_velocity_maxima": [vp, i, dp],
@@ -123,6 +127,52 @@ def _check(rc: int):
 
 def _fptr(a: np.ndarray):
     return a.ctypes.data_as(C.c_void_p)
+
+
+class _ResultBuffers:
+    """Page-locked host memory for large results, so that they arrive by one
+    direct copy instead of through the driver's staging and the first touch of
+    new pages (10.5 MB of a predictor gradient: 0.2 ms against 1.3). An array
+    made here is the caller's; its memory comes back when the last view of it
+    is gone. At most LIMIT bytes are held, in use or waiting; past that, and
+    for results under SMALL bytes, the array is ordinary memory."""
+    LIMIT, SMALL = 64 << 20, 1 << 18
+
+    def __init__(self):
+        self.lock = threading.Lock()
+        self.held = 0
+        self.free = {}                         # bytes -> [address]
+        self.returned = collections.deque()    # (address, bytes), put here by finalizers without the lock
+
+    def _take(self, nbytes):
+        with self.lock:
+            while self.returned:
+                ptr, n = self.returned.popleft()
+                self.free.setdefault(n, []).append(ptr)
+            if self.free.get(nbytes):
+                return self.free[nbytes].pop()
+            for size, ptrs in list(self.free.items()):   # buffers of other sizes make room
+                while ptrs and self.held + nbytes > self.LIMIT:
+                    load_library().sf_host_free(C.c_void_p(ptrs.pop()))
+                    self.held -= size
+            p = C.c_void_p()
+            if self.held + nbytes > self.LIMIT or load_library().sf_host_alloc(nbytes, C.byref(p)) != 0:
+                return None
+            self.held += nbytes
+            return p.value
+
+    def empty(self, shape):
+        """A float32 array of unset values."""
+        n = int(np.prod(shape))
+        ptr = self._take(4 * n) if 4 * n >= self.SMALL else None
+        if ptr is None:
+            return np.zeros(shape, dtype=np.float32)
+        raw = (C.c_float * n).from_address(ptr)
+        weakref.finalize(raw, self.returned.append, (ptr, 4 * n)).atexit = False
+        return np.frombuffer(raw, dtype=np.float32).reshape(shape)
+
+
+_results = _ResultBuffers()
 
 
 class IMEXRK:
@@ -682,7 +732,7 @@ class Net:
         x = np.ascontiguousarray(x, dtype=np.float32)
         B = x.shape[0]
         assert x.shape == (B, self.Z, self.channels[0])
-        y = np.zeros((B, self.Z, self.channels[-1]), dtype=np.float32)
+        y = _results.empty((B, self.Z, self.channels[-1]))
         _check(load_library().sf_net_forward(self._h, _fptr(x), B, _fptr(y)))
         return y
 
@@ -695,7 +745,7 @@ class Net:
         _check(load_library().sf_net_set_data(self._h, _fptr(x), _fptr(target), B))
 
     def gradient(self):
-        g = np.zeros(self.num_params, dtype=np.float32)
+        g = _results.empty((self.num_params,))
         loss = C.c_double()
         _check(load_library().sf_net_gradient(self._h, _fptr(g), C.byref(loss)))
         return g, loss.value

@@ -526,10 +526,11 @@ int upload_input(sf_net* n, const float* x, int B) {
 
 extern "C" {
 
-// after a synchronisation: a GEMM whose tensor-core wait ran out is an error
+// waits for the stream; a GEMM whose tensor-core wait ran out is an error
 static int net_status(sf_net* n) {
   int h = 0;
-  NCK(cudaMemcpy(&h, n->err, sizeof(int), cudaMemcpyDeviceToHost));
+  NCK(cudaMemcpyAsync(&h, n->err, sizeof(int), cudaMemcpyDeviceToHost, n->st));
+  NCK(cudaStreamSynchronize(n->st));
   if (h) {
     NCK(cudaMemset(n->err, 0, sizeof(int)));
     return nfail(SF_ECUDA, "a tensor-core GEMM block gave up waiting for its MMAs");
@@ -661,7 +662,6 @@ int sf_net_forward(sf_net* n, const float* x, int batch, float* y) {
   if (rc) return rc;
   n->nb_data = 0;   // act[0] no longer holds the training inputs
   NCK(cudaMemcpyAsync(y, n->out, sizeof(float) * batch * n->Z * n->ch[n->nl], cudaMemcpyDeviceToHost, n->st));
-  NCK(cudaStreamSynchronize(n->st));
   return net_status(n);
 }
 
@@ -682,7 +682,6 @@ int sf_net_gradient(sf_net* n, float* grad, double* loss) {
   if (rc) return rc;
   if (grad) NCK(cudaMemcpyAsync(grad, n->gr, sizeof(float) * n->nparam, cudaMemcpyDeviceToHost, n->st));
   if (loss) NCK(cudaMemcpyAsync(loss, n->loss, sizeof(double), cudaMemcpyDeviceToHost, n->st));
-  NCK(cudaStreamSynchronize(n->st));
   return net_status(n);
 }
 
@@ -702,7 +701,6 @@ int sf_net_train(sf_net* n, int steps, double lr, double* losses) {
     if (rc) return rc;
     if (losses) NCK(cudaMemcpyAsync(losses + s, n->loss, sizeof(double), cudaMemcpyDeviceToHost, n->st));
   }
-  NCK(cudaStreamSynchronize(n->st));
   return net_status(n);
 }
 
