@@ -241,4 +241,117 @@ __device__ __forceinline__ void reg_fft2_256w(c2x (&x)[8], float4* buf, const fl
   }
 }
 
+// The packed transform pair of N = 128 points over 16 lanes (8 points each) in
+// three stages: as reg_fft2_256w with 16 = 4 x 4 in place of 32 = 8 x 4: an
+// 8-point DFT over e and W_128^{l k1} (w1); lane l takes column k1 = l % 8 at
+// l0 = l / 8 + 2 h, h = 0, 1, for the 4-point DFTs over l1 and W_16^{l0 m};
+// then the values l0 = 0..3 of (k1 = l % 8, m = l / 8 + 2 i), i = 0, 1, for two
+// 4-point DFTs. On exit slot i*4 + q holds out[l + 16 j] with j = i + 2 q. buf
+// holds 8 x 17 float4 per group. Eight points a lane instead of sixteen (the
+// two-stage form over 8 lanes) is half the registers, twice the warps.
+__device__ __forceinline__ void fill_tw2_128h(float4* tw4, float2* tw2, const float2* __restrict__ tw, int tid,
+                                              int nthr) {
+  for (int i = tid; i < 8 * 16; i += nthr) {
+    const int k1 = i / 16, l = i - k1 * 16;
+    const float2 w = tw[(l * k1) * (kMaxN / 128)];
+    tw4[i] = make_float4(w.x, w.x, w.y, w.y);
+  }
+  float4* t2 = reinterpret_cast<float4*>(tw2);
+  for (int i = tid; i < 4 * 4; i += nthr) {
+    const int m = i / 4, l0 = i - m * 4;
+    const float2 w = tw[(8 * l0 * m) * (kMaxN / 128)];
+    t2[i] = make_float4(w.x, w.x, w.y, w.y);
+  }
+}
+template <bool INV>
+__device__ __forceinline__ void reg_fft2_128h(c2x (&x)[8], float4* buf, const float2* __restrict__ tw2, int l,
+                                              const float4 (&w1)[8]) {
+  dft2<8, INV>(x);
+#pragma unroll
+  for (int k1 = 1; k1 < 8; k1++) x[k1] = tw2_mul_reg<INV>(x[k1], w1[k1]);
+  __syncwarp();
+#pragma unroll
+  for (int k1 = 0; k1 < 8; k1++) buf[k1 * 17 + l] = c2x_to4(x[k1]);    // element (row l, column k1)
+  __syncwarp();
+  const int k1 = l & 7, a = l >> 3;
+#pragma unroll
+  for (int h = 0; h < 2; h++)
+#pragma unroll
+    for (int l1 = 0; l1 < 4; l1++) x[h * 4 + l1] = c2x_of4(buf[k1 * 17 + a + 2 * h + 4 * l1]);
+  __syncwarp();
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    dft2<4, INV>(x + 4 * h);
+#pragma unroll
+    for (int m = 1; m < 4; m++)
+      tw2_apply<INV>(x[h * 4 + m], reinterpret_cast<const float4*>(tw2) + m * 4 + a + 2 * h, tw2);
+  }
+#pragma unroll
+  for (int i = 0; i < 8; i++) buf[i * 17 + l] = c2x_to4(x[i]);         // element (lane l, h*4 + m)
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 2; i++)
+#pragma unroll
+    for (int l0 = 0; l0 < 4; l0++) x[i * 4 + l0] = c2x_of4(buf[((l0 >> 1) * 4 + a + 2 * i) * 17 + k1 + 8 * (l0 & 1)]);
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 2; i++) dft2<4, INV>(x + 4 * i);
+}
+
+// The packed transform pair of N = 512 points over a whole warp (32 lanes,
+// 16 points each): as reg_fft2_256w with 16 columns k1: a 16-point DFT over e
+// and W_512^{l k1} (tw4, [k1][l]); lane l takes columns k1 = l % 16 at l0 = l /
+// 16 + 2 h, h = 0, 1, for the 8-point DFTs over l1 and W_32^{l0 m}; then the
+// values l0 = 0..3 of (k1 = l % 16, m = l / 16 + 2 i), i < 4, for four 4-point
+// DFTs. On exit slot i*4 + q holds out[l + 32 j] with j = i + 4 q. buf holds 16
+// x 33 float4.
+__device__ __forceinline__ void fill_tw2_512w(float4* tw4, float2* tw2, const float2* __restrict__ tw, int tid,
+                                              int nthr) {
+  for (int i = tid; i < 16 * 32; i += nthr) {
+    const int k1 = i / 32, l = i - k1 * 32;
+    const float2 w = tw[(l * k1) * (kMaxN / 512)];
+    tw4[i] = make_float4(w.x, w.x, w.y, w.y);
+  }
+  float4* t2 = reinterpret_cast<float4*>(tw2);
+  for (int i = tid; i < 8 * 4; i += nthr) {
+    const int m = i / 4, l0 = i - m * 4;
+    const float2 w = tw[(16 * l0 * m) * (kMaxN / 512)];
+    t2[i] = make_float4(w.x, w.x, w.y, w.y);
+  }
+}
+template <bool INV>
+__device__ __forceinline__ void reg_fft2_512w(c2x (&x)[16], float4* buf, const float4* __restrict__ tw4,
+                                              const float2* __restrict__ tw2, int l) {
+  dft2<16, INV>(x);
+#pragma unroll
+  for (int k1 = 1; k1 < 16; k1++) tw2_apply<INV>(x[k1], tw4 + k1 * 32 + l, tw2);
+  __syncwarp();
+#pragma unroll
+  for (int k1 = 0; k1 < 16; k1++) buf[k1 * 33 + l] = c2x_to4(x[k1]);   // element (row l, column k1)
+  __syncwarp();
+  const int k1 = l & 15, a = l >> 4;
+#pragma unroll
+  for (int h = 0; h < 2; h++)
+#pragma unroll
+    for (int l1 = 0; l1 < 8; l1++) x[h * 8 + l1] = c2x_of4(buf[k1 * 33 + a + 2 * h + 4 * l1]);
+  __syncwarp();
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    dft2<8, INV>(x + 8 * h);
+#pragma unroll
+    for (int m = 1; m < 8; m++)
+      tw2_apply<INV>(x[h * 8 + m], reinterpret_cast<const float4*>(tw2) + m * 4 + a + 2 * h, tw2);
+  }
+#pragma unroll
+  for (int i = 0; i < 16; i++) buf[i * 33 + l] = c2x_to4(x[i]);        // element (lane l, h*8 + m)
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+#pragma unroll
+    for (int l0 = 0; l0 < 4; l0++) x[i * 4 + l0] = c2x_of4(buf[((l0 >> 1) * 8 + a + 2 * i) * 33 + k1 + 16 * (l0 & 1)]);
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 4; i++) dft2<4, INV>(x + 4 * i);
+}
+
 }  // namespace sf

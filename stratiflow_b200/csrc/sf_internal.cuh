@@ -143,11 +143,16 @@ int prepare_zstep_tma_kernels();
 bool zstep_f_supported(const Geo& g);
 int launch_z_step_f(const StageArgs& a, cudaStream_t st);
 int prepare_zstep_f_kernels();
-// the 3D nonlinear x pass as level-marching lane groups (sf_xmarch.cu): levels
-// t_lo .. t_hi - 1 of every run and y row
-bool xmarch_supported(const StageArgs& a);
-int launch_xmarch(const StageArgs& a, int t_lo, int t_hi, cudaStream_t st);
+// the x pass as level-marching lane groups (sf_xmarch.cu): levels t_lo ..
+// t_hi - 1 of every y row of runs a.run_offset .. + nruns - 1; mode 0
+// BuildRHS, 1 BuildRHSLinear about the frozen base, 2 about the live base run
+bool xmarch_supported(const StageArgs& a, int mode, int nruns);
+int launch_xmarch(const StageArgs& a, int mode, int nruns, int t_lo, int t_hi, cudaStream_t st);
 int prepare_xmarch_kernels();
+// the adjoint x pass in the same manner (sf_adjmarch.cu): every level of every run
+bool adjmarch_supported(const Geo& g);
+int launch_adjmarch(const StageArgs& a, cudaStream_t st);
+int prepare_adjmarch_kernels();
 // one stage; if ev != nullptr, ev[i] is recorded after the i-th kernel
 int launch_stage(const StageArgs& a, cudaStream_t st, cudaEvent_t* ev = nullptr, const XYAux* aux = nullptr);
 int stage_kernel_count(const Geo& g);

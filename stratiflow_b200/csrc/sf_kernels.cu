@@ -1410,27 +1410,34 @@ static void launch_xpass_runs(const StageArgs& a, bool L, int nruns, cudaStream_
   }
 }
 
+// the x pass of runs run0 .. + nruns - 1, mode as launch_xmarch's: the level
+// march where the setting and the grid take it, else the slab kernel
+static void launch_xpass_mode(const StageArgs& a, int mode, int run0, int nruns, cudaStream_t st) {
+  StageArgs b = a;
+  b.run_offset = run0;
+  if (a.xkernel == 1 && xmarch_supported(a, mode, nruns)) {
+    // the same level columns as the slab kernel's launch would cover
+    int lo = 0, hi = a.g.N3;
+    if (a.xcols > 0 || a.xcol0 > 0) {
+      const int lv = xpass_column_levels(a, mode != 0, a.g.nrun);
+      lo = a.xcol0 * lv;
+      if (a.xcols > 0) hi = std::min(hi, (a.xcol0 + a.xcols) * lv);
+    }
+    launch_xmarch(b, mode, nruns, lo, hi, st);
+    return;
+  }
+  launch_xpass_runs(b, mode != 0, nruns, st);
+}
+
 // the x pass of every run: one launch, or for a tangent-linear batch one
 // nonlinear launch for the base runs and one linear launch for the rest
 static int launch_xpass(const StageArgs& a, cudaStream_t st) {
   if (a.tlm > 0) {
-    StageArgs b = a;
-    b.run_offset = 0;
-    launch_xpass_runs(b, false, a.tlm, st);
-    b.run_offset = a.tlm;
-    launch_xpass_runs(b, true, a.g.nrun - a.tlm, st);
+    launch_xpass_mode(a, 0, 0, a.tlm, st);
+    launch_xpass_mode(a, 2, a.tlm, a.g.nrun - a.tlm, st);
     return 2;
   }
-  StageArgs b = a;
-  b.run_offset = 0;
-  if (a.xkernel == 1 && xmarch_supported(a)) {
-    // the same level columns as the slab kernel's launch would cover
-    const int lv = xpass_column_levels(a, false, a.g.nrun);
-    const int ncol = (int)cdiv(a.g.N3, lv);
-    const int c1 = a.xcols > 0 ? a.xcol0 + a.xcols : ncol;
-    return launch_xmarch(b, a.xcol0 * lv, std::min(a.g.N3, c1 * lv), st);
-  }
-  launch_xpass_runs(b, a.linear != 0, a.g.nrun, st);
+  launch_xpass_mode(a, a.linear ? 1 : 0, 0, a.g.nrun, st);
   return 1;
 }
 

@@ -801,8 +801,8 @@ int sf_profile_step(sf_solver* s, int nsteps, int linear, int cap, double* ms, i
 int sf_profile_names(sf_solver* s, char* buf, size_t len) {
   if (!s || !buf || len == 0) return fail(SF_EINVAL, "bad argument");
   std::string out;
-  // the nonlinear 3D x pass runs as k_xmarch where the solver takes it
-  const bool march = s->xkernel == 1 && !s->tlm && xmarch_supported(stage_args(s, 0, s->cur, false));
+  // the x pass runs as k_xmarch where the solver takes it
+  const bool march = s->xkernel == 1 && xmarch_supported(stage_args(s, 0, s->cur, false), s->tlm ? 2 : 0, s->g.nrun - s->tlm);
   // and the z pass as k_z_step_tma
   const StageArgs a0 = stage_args(s, 0, s->cur, false);
   const char* zname = z_step_takes_c(a0) ? (zstep_f_supported(a0.g) ? "k_z_step_f" : "k_z_step_c") : (z_step_takes_tma(a0) ? "k_z_step_tma" : "k_z_step");
