@@ -644,6 +644,7 @@ int prepare_adjoint_kernels() {
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_xpass_adj3<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   ADJ_ATTR(16) ADJ_ATTR(32) ADJ_ATTR(64) ADJ_ATTR(128) ADJ_ATTR(256) ADJ_ATTR(512)
 #undef ADJ_ATTR
+  if (e == cudaSuccess && prepare_adjmarch_kernels() != 0) return -1;
   return e == cudaSuccess ? 0 : -1;
 }
 
@@ -663,7 +664,8 @@ int launch_stage_adjoint(StageArgs a, const float2* below, const float2* above, 
       case 128: ify_adj_launch<128>(a, st); break;
       case 256: ify_adj_launch<256>(a, st); break;
     }
-    switch (g.N1) {
+    if (a.xkernel == 1 && adjmarch_supported(g)) launch_adjmarch(a, st);
+    else switch (g.N1) {
       case 16: adj3_launch<16>(a, st); break;
       case 32: adj3_launch<32>(a, st); break;
       case 64: adj3_launch<64>(a, st); break;
@@ -674,7 +676,8 @@ int launch_stage_adjoint(StageArgs a, const float2* below, const float2* above, 
     launch_fft_y_combos(a, st);
     return 4 + launch_z_solves(a, st);
   }
-  switch (g.N1) {
+  if (a.xkernel == 1 && adjmarch_supported(g)) launch_adjmarch(a, st);
+  else switch (g.N1) {
     case 16: adj_launch<16>(a, st); break;
     case 32: adj_launch<32>(a, st); break;
     case 64: adj_launch<64>(a, st); break;
