@@ -216,13 +216,14 @@ int sf_set_z_kernel(sf_solver* s, int kind);
  * on it. */
 int sf_set_xpass_groups(sf_solver* s, int groups);
 
-/* Launch tuning of the 3D nonlinear x pass (no counterpart in the reference):
- * kind 1 (the default) runs it as lane groups that each own a y row and
- * march up a range of levels, transforming two fields or products per packed
- * FP32 instruction; kind 0 as blocks over slabs of levels (the kernel that
- * every other x pass uses). The results agree to rounding (the z stencils'
- * terms are summed in another order). Grids with N1 other than 64, 128 or 256
- * always take kind 0. */
+/* Launch tuning of the x pass (no counterpart in the reference): kind 1 (the
+ * default) runs it (nonlinear, linear, tangent-linear and adjoint) as lane
+ * groups that each own a row and march up a range of levels, transforming two
+ * fields or products per packed FP32 instruction; kind 0 as blocks over slabs
+ * of levels. The results agree to rounding (the z stencils' terms are summed
+ * in another order). 3D grids with N1 other than 64, 128 or 256, small 2D
+ * launches (under 2^18 points, except the frozen-base step) and the 2D adjoint
+ * outside N1 = 32 .. 256 always take kind 0. */
 int sf_set_xpass_kernel(sf_solver* s, int kind);
 
 /* IMEXRK::KE / PE (IMEXRK.h:395-411) of one run, accumulated in FP64 */

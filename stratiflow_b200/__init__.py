@@ -456,8 +456,9 @@ class IMEXRK:
         _check(load_library().sf_set_xpass_groups(self._h, int(groups)))
 
     def set_xpass_kernel(self, kind):
-        """3D nonlinear x pass: 1 level-marching lane groups (default), 0 slab
-        blocks; a launch setting (the results change only by rounding)."""
+        """x pass: 1 level-marching lane groups (default, where the grid takes
+        them), 0 slab blocks; a launch setting (the results change only by
+        rounding)."""
         _check(load_library().sf_set_xpass_kernel(self._h, int(kind)))
 
     def set_z_kernel(self, kind):

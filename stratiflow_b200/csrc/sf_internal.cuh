@@ -117,13 +117,13 @@ struct XYAux {
   int bands;
 };
 
-// one block's work in an ensemble launch: member solver `run`, block
-// coordinate x (x-pass level column or z-solve mode group), and for the x
-// pass the slab height S and slabs per block
+// one block's work in an ensemble launch: member solver `run`; x pass: units x
+// .. x + iters - 1 (one per warp) of segments of S levels; z: mode group x
 struct EnsItem {
   int run, x, S, iters;
 };
-constexpr int kEnsThreads = 256;
+constexpr int kEnsThreads = 384;
+constexpr int kEnsFusedN3 = 484;   // the tallest column of a z item in k_z_step_f's shape of 12 warps
 
 // launchers (sf_kernels.cu); each returns the number of kernels launched
 int prepare_kernels();
@@ -173,20 +173,18 @@ int launch_gather_ref(const Geo& g, const float2* ref, float2* kept, cudaStream_
 int launch_scatter_ref(const Geo& g, const float2* kept, float2* ref, cudaStream_t st);
 int launch_energy(const Geo& g, const float2* Sa, const float2* Sb, int nrun_pairs,
                   const float* zc, const float* Ri, double* out, cudaStream_t st);
-// ensembles of 2D solvers of different grids (sf_ensemble): every member's
-// x pass in one launch and every member's z step in another; args holds one
-// StageArgs per member
-size_t ensemble_xpass_smem(int N1, int S);
-size_t ensemble_zstep_smem(int N3);
-int launch_xpass_ens(const StageArgs* args, const EnsItem* items, int nitems, size_t smem, cudaStream_t st);
-int launch_zstep_ens(const StageArgs* args, const EnsItem* items, int nitems, size_t smem, cudaStream_t st);
+// ensembles of 2D solvers of different grids (sf_ens.cu): one stage of every
+// member in one launch of `blocks` persistent blocks over work-item counters
+// (counters[0] the next item, counters[1 + r] member r's finished x items;
+// cleared before each step); args holds one StageArgs per member
+int ensemble_z_modes(int N3);
+int ensemble_x_warps(int N1);
+int ensemble_x_rows(int N1);
+size_t ensemble_smem(int N1, int N3);
 int prepare_ensemble_kernels();
-// the whole stage in one launch of `blocks` persistent blocks over work-item
-// counters (counters[0] the next item, counters[1 + r] member r's finished
-// x-pass items; cleared before each step)
 int launch_ens_stage(const StageArgs* args, const EnsItem* xitems, int nx, const EnsItem* zitems, int nz,
                      int* counters, const int* xneed, int* err, int blocks, size_t smem, cudaStream_t st);
-int ensemble_stage_blocks(size_t smem);
+int ensemble_stage_blocks();
 int launch_grad_sq(const Geo& g, const float2* S, int nruns, const float* zc, const double* kxd, const double* kyd,
                    double* out, cudaStream_t st);
 int launch_base_nodal(const Geo& g, const float2* kept_modal, int field, float* base_out,

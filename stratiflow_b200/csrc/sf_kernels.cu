@@ -1035,122 +1035,6 @@ __global__ void __launch_bounds__(ZW * 32, ZW == 8 ? 3 : 1) k_z_step(StageArgs a
 }
 
 
-// ============================================================ ensembles ====
-// Every member of an ensemble of 2D solvers (grids of different sizes, one
-// run each) in one launch per kernel: a block reads its work item and its
-// member's stage arguments and runs the same block body as the solver's own
-// launch would. Blocks have kEnsThreads threads for every grid; the dynamic
-// shared memory is the largest any member needs.
-__global__ void __launch_bounds__(kEnsThreads, 2) k_xpass_ens(const StageArgs* __restrict__ args,
-                                                              const EnsItem* __restrict__ items) {
-  __shared__ StageArgs sa;
-  const EnsItem it = items[blockIdx.x];
-  if (threadIdx.x == 0) sa = args[it.run];
-  __syncthreads();
-  switch (sa.g.N1) {
-    case 16: xpass_body<16, false>(sa, it.S, it.iters, it.x, 0, 0); break;
-    case 32: xpass_body<32, false>(sa, it.S, it.iters, it.x, 0, 0); break;
-    case 64: xpass_body<64, false>(sa, it.S, it.iters, it.x, 0, 0); break;
-    case 128: xpass_body<128, false>(sa, it.S, it.iters, it.x, 0, 0); break;
-    case 256: xpass_body<256, false>(sa, it.S, it.iters, it.x, 0, 0); break;
-    case 512: xpass_body<512, false>(sa, it.S, it.iters, it.x, 0, 0); break;
-    default: break;
-  }
-}
-
-__global__ void __launch_bounds__(kEnsThreads, 2) k_zstep_ens(const StageArgs* __restrict__ args,
-                                                              const EnsItem* __restrict__ items) {
-  __shared__ StageArgs sa;
-  const EnsItem it = items[blockIdx.x];
-  if (threadIdx.x == 0) sa = args[it.run];
-  __syncthreads();
-  if (sa.zkernel == 2 && zc_fits(sa.g.N3)) z_step_c_body<kCC, true>(sa, it.x, 0);
-  else if ((sa.g.N3 + 7) / 8 >= 48) z_step_body<8, true>(sa, it.x, 0);
-  else z_step_body<8, false>(sa, it.x, 0);
-}
-
-
-// One RK stage of every member in one launch: blocks claim work items from
-// counters[0] in order, all x-pass items first (largest members first), then
-// all z-step items. A z-step item of member r starts once member r's x-pass
-// items have all finished (counters[1 + r] reaches xneed[r]). A block claims
-// its next item as it starts the current one, so the claim's latency hides
-// behind the work; every wait still ends: an item claimed ahead always has a
-// higher index than the claiming block's current item, so every x-pass item
-// is being run or is next after an x-pass item being run, and x-pass items
-// wait on nothing. The waits are bounded all the same: one that runs out
-// sets *err and skips its item. The host clears the counters before each step.
-constexpr long long kEnsSpin = 1ll << 24;   // x 64 ns: about a second
-
-__global__ void __launch_bounds__(kEnsThreads, 2) k_ens_stage(const StageArgs* __restrict__ args,
-                                                              const EnsItem* __restrict__ xitems, int nx,
-                                                              const EnsItem* __restrict__ zitems, int nz,
-                                                              int* counters, const int* __restrict__ xneed,
-                                                              int* err) {
-  __shared__ __align__(16) StageArgs sa;
-  __shared__ int next, have, ok;
-  static_assert(sizeof(StageArgs) % sizeof(int) == 0, "StageArgs copied as words");
-  if (threadIdx.x == 0) {
-    next = atomicAdd(&counters[0], 1);
-    have = -1;
-  }
-  __syncthreads();
-  for (;;) {
-    const int i = next;
-    if (i >= nx + nz) break;
-    const bool xp = i < nx;
-    const EnsItem it = xp ? xitems[i] : zitems[i - nx];
-    const bool fresh = it.run != have;
-    __syncthreads();   // everyone has read next and have
-    if (threadIdx.x == 0) {
-      next = atomicAdd(&counters[0], 1);
-      have = it.run;
-      ok = 1;
-    }
-    if (fresh) {   // this member's stage arguments, copied by the block's threads
-      const int* src = reinterpret_cast<const int*>(args + it.run);
-      int* dst = reinterpret_cast<int*>(&sa);
-      for (int w = threadIdx.x; w < (int)(sizeof(StageArgs) / sizeof(int)); w += blockDim.x) dst[w] = src[w];
-    }
-    if (!xp && threadIdx.x == 0) {
-      const volatile int* done = counters + 1 + it.run;
-      long long n = 0;
-      while (*done < xneed[it.run] && n < kEnsSpin) {
-        __nanosleep(64);
-        n++;
-      }
-      if (*done < xneed[it.run]) {
-        ok = 0;
-        atomicExch(err, 1);
-      }
-      __threadfence();   // the member's x-pass results before its z step reads them
-    }
-    __syncthreads();
-    if (xp) {
-      switch (sa.g.N1) {
-        case 16: xpass_body<16, false>(sa, it.S, it.iters, it.x, 0, 0); break;
-        case 32: xpass_body<32, false>(sa, it.S, it.iters, it.x, 0, 0); break;
-        case 64: xpass_body<64, false>(sa, it.S, it.iters, it.x, 0, 0); break;
-        case 128: xpass_body<128, false>(sa, it.S, it.iters, it.x, 0, 0); break;
-        case 256: xpass_body<256, false>(sa, it.S, it.iters, it.x, 0, 0); break;
-        case 512: xpass_body<512, false>(sa, it.S, it.iters, it.x, 0, 0); break;
-        default: break;
-      }
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        __threadfence();   // this item's r rows, before it counts as done
-        atomicAdd(&counters[1 + it.run], 1);
-      }
-    } else if (ok) {   // the member's own z kernel: one lane per complex mode, or one per component
-      if (sa.zkernel == 2 && zc_fits(sa.g.N3)) z_step_c_body<kCC, true>(sa, it.x, 0);
-      else if ((sa.g.N3 + 7) / 8 >= 48) z_step_body<8, true>(sa, it.x, 0);
-      else z_step_body<8, false>(sa, it.x, 0);
-    }
-    __syncthreads();
-  }
-}
-
-
 // ====================================================== factorisation ====
 // Thomas factors of every (factor set, mode) in FP64 (Tridiagonal.h:14-27):
 // inv_den_j = 1/(b_j - a_j C_{j-1}), stored as float. Rows follow
@@ -1415,7 +1299,9 @@ static void launch_xpass_runs(const StageArgs& a, bool L, int nruns, cudaStream_
 static void launch_xpass_mode(const StageArgs& a, int mode, int run0, int nruns, cudaStream_t st) {
   StageArgs b = a;
   b.run_offset = run0;
-  if (a.xkernel == 1 && xmarch_supported(a, mode, nruns)) {
+  // the base runs of a tangent-linear batch take the kernel that a plain batch
+  // of its size takes, so that they stay bit for bit what they are there
+  if (a.xkernel == 1 && xmarch_supported(a, mode, mode == 0 ? a.g.nrun : nruns)) {
     // the same level columns as the slab kernel's launch would cover
     int lo = 0, hi = a.g.N3;
     if (a.xcols > 0 || a.xcol0 > 0) {
@@ -1652,54 +1538,6 @@ int launch_gather_ref(const Geo& g, const float2* ref, float2* kept, cudaStream_
 int launch_scatter_ref(const Geo& g, const float2* kept, float2* ref, cudaStream_t st) {
   k_scatter_ref<<<dim3(cdiv(g.P, 32), cdiv(g.N3, 32)), dim3(32, 8), 0, st>>>(g, kept, ref);
   return 1;
-}
-
-static int fft_G(int N) { return N >= 256 ? 16 : (N >= 64 ? 8 : 4); }
-static int fft_bufstride(int N) {
-  switch (N) {
-    case 16: return fft_buf_stride<16>();
-    case 32: return fft_buf_stride<32>();
-    case 64: return fft_buf_stride<64>();
-    case 128: return fft_buf_stride<128>();
-    case 256: return fft_buf_stride<256>();
-    default: return fft_buf_stride<512>();
-  }
-}
-
-size_t ensemble_xpass_smem(int N1, int S) {
-  return x_layout(S, N1, N1 / 3, 0, 0, fft_bufstride(N1), kEnsThreads / fft_G(N1), 0, 0).bytes;
-}
-size_t ensemble_zstep_smem(int N3) {
-  return std::max(sizeof(float) * ((size_t)N3 * 32 + 3 * 8 * 32), zc_smem_bytes(N3));
-}
-
-int launch_xpass_ens(const StageArgs* args, const EnsItem* items, int nitems, size_t smem, cudaStream_t st) {
-  k_xpass_ens<<<nitems, kEnsThreads, smem, st>>>(args, items);
-  return 1;
-}
-int launch_zstep_ens(const StageArgs* args, const EnsItem* items, int nitems, size_t smem, cudaStream_t st) {
-  k_zstep_ens<<<nitems, kEnsThreads, smem, st>>>(args, items);
-  return 1;
-}
-int launch_ens_stage(const StageArgs* args, const EnsItem* xitems, int nx, const EnsItem* zitems, int nz,
-                     int* counters, const int* xneed, int* err, int blocks, size_t smem, cudaStream_t st) {
-  k_ens_stage<<<blocks, kEnsThreads, smem, st>>>(args, xitems, nx, zitems, nz, counters, xneed, err);
-  return 1;
-}
-int ensemble_stage_blocks(size_t smem) {
-  int per_sm = 0, sms = 0, dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ens_stage, kEnsThreads, smem) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-    return 148;
-  return (per_sm < 1 ? 1 : per_sm) * sms;
-}
-int prepare_ensemble_kernels() {
-  const int lim = 227 * 1024 - (int)sizeof(StageArgs) - 64;
-  cudaError_t e = cudaFuncSetAttribute(k_xpass_ens, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_zstep_ens, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_ens_stage, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-  return e == cudaSuccess ? 0 : -1;
 }
 
 int launch_grad_sq(const Geo& g, const float2* S, int nruns, const float* zc, const double* kxd, const double* kyd,

@@ -6,6 +6,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -301,6 +302,17 @@ const float2* sf_solver_tw(const sf_solver* s) { return s->tw; }
 const float* sf_solver_ubar(const sf_solver* s, int run) { return s->Ubar + (size_t)run * s->g.N3; }
 void sf_solver_count_launches(sf_solver* s, int n) { s->launches += n; }
 
+// the kernels' shared-memory limits, set once per device (the current one)
+static bool kernels_ready(int device) {
+  static std::mutex mu;
+  static std::vector<int> done;
+  std::lock_guard<std::mutex> lock(mu);
+  if (std::find(done.begin(), done.end(), device) != done.end()) return true;
+  if (prepare_kernels() != 0 || prepare_adjoint_kernels() != 0) return false;
+  done.push_back(device);
+  return true;
+}
+
 extern "C" {
 
 const char* sf_last_error(void) { return g_err.c_str(); }
@@ -345,8 +357,7 @@ int sf_create(const sf_grid* grid, const sf_flow* flow, double dt, int device, s
     }                                                                                              \
   } while (0)
 
-  if (prepare_kernels() != 0 || prepare_adjoint_kernels() != 0)
-    return cleanup_fail(fail(SF_ECUDA, "cudaFuncSetAttribute failed"));
+  if (!kernels_ready(device)) return cleanup_fail(fail(SF_ECUDA, "cudaFuncSetAttribute failed"));
   CKC(cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking));
   if (g.dim3) {
     CKC(cudaStreamCreateWithFlags(&s->xy.y1, cudaStreamNonBlocking));
@@ -978,11 +989,12 @@ struct sf_ensemble {
   cudaStream_t st = nullptr;
   StageArgs* d_args = nullptr;   // [parity][stage][member]
   std::vector<StageArgs> h_args;
+  bool args_set = false;         // d_args holds h_args
   EnsItem *d_x = nullptr, *d_z = nullptr;
   int nx = 0, nz = 0;
-  size_t xsmem = 0, zsmem = 0;
+  size_t smem = 0;
   int* d_counters = nullptr;   // [3 stages][1 + nrun] work-item counters of the stage launches
-  int* d_xneed = nullptr;      // [nrun] x-pass items per member
+  int* d_xneed = nullptr;      // [nrun] x-pass items per member, then nrun zeros
   int* d_err = nullptr;        // a z-step item whose wait ran out
   int blocks = 0;              // persistent blocks of a stage launch
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
@@ -1023,23 +1035,42 @@ int sf_ensemble_create(int nrun, const sf_grid* grids, const sf_flow* flows, con
     }
     e->members.push_back(m);
   }
-  // work items, the largest members first; every x-pass block takes one
-  // 4-level slab (S = 4, no carried slabs)
+  // work items, the largest members first. An x item is 12 warps' worth of
+  // segments; a segment of n levels costs n + 1.7 (its first level's and its
+  // last's extra transforms), so the segments are as long as still leaves
+  // items for every SM
   std::vector<int> order(nrun);
   for (int r = 0; r < nrun; r++) order[r] = r;
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
     return (long long)grids[a].N1 * grids[a].N3 > (long long)grids[b].N1 * grids[b].N3;
   });
+  e->blocks = ensemble_stage_blocks();
+  auto units = [&](const Geo& g, int seg) {
+    const int W = ensemble_x_rows(g.N1);
+    return ((g.N3 + seg - 1) / seg + W - 1) / W;
+  };
+  int seg = 1;
+  double best = 1e300;
+  for (int n = 1; n <= 8; n++) {
+    long long items = 0;
+    for (int r = 0; r < nrun; r++) {
+      const Geo& g = e->members[r]->g;
+      items += (units(g, n) + ensemble_x_warps(g.N1) - 1) / ensemble_x_warps(g.N1);
+    }
+    const double rounds = (double)items / e->blocks, t = (rounds > 1 ? rounds + 0.5 : 1.0) * (n + 1.7);
+    if (t < best) {
+      best = t;
+      seg = n;
+    }
+  }
   std::vector<EnsItem> xi, zi;
-  std::vector<int> xneed(nrun, 0);
+  std::vector<int> xneed(2 * nrun, 0);
   for (int r : order) {
     const Geo& g = e->members[r]->g;
-    const int S = 4;
-    xneed[r] = (g.N3 + S - 1) / S;
-    for (int c = 0; c < (g.N3 + S - 1) / S; c++) xi.push_back(EnsItem{r, c, S, 1});
-    for (int q = 0; q < (g.P + 15) / 16; q++) zi.push_back(EnsItem{r, q, 0, 0});
-    e->xsmem = std::max(e->xsmem, ensemble_xpass_smem(g.N1, S));
-    e->zsmem = std::max(e->zsmem, ensemble_zstep_smem(g.N3));
+    const int U = units(g, seg), nw = ensemble_x_warps(g.N1), zm = ensemble_z_modes(g.N3);
+    for (int u = 0; u < U; u += nw, xneed[r]++) xi.push_back(EnsItem{r, u, seg, std::min(nw, U - u)});
+    for (int q = 0; q < (g.P + zm - 1) / zm; q++) zi.push_back(EnsItem{r, q, 0, 0});
+    e->smem = std::max(e->smem, ensemble_smem(g.N1, g.N3));
   }
   e->nx = (int)xi.size();
   e->nz = (int)zi.size();
@@ -1050,16 +1081,15 @@ int sf_ensemble_create(int nrun, const sf_grid* grids, const sf_flow* flows, con
   if (ce == cudaSuccess) ce = cudaMemcpy(e->d_x, xi.data(), sizeof(EnsItem) * xi.size(), cudaMemcpyHostToDevice);
   if (ce == cudaSuccess) ce = cudaMemcpy(e->d_z, zi.data(), sizeof(EnsItem) * zi.size(), cudaMemcpyHostToDevice);
   if (ce == cudaSuccess) ce = cudaMalloc(&e->d_counters, sizeof(int) * 3 * (nrun + 1));
-  if (ce == cudaSuccess) ce = cudaMalloc(&e->d_xneed, sizeof(int) * nrun);
+  if (ce == cudaSuccess) ce = cudaMalloc(&e->d_xneed, sizeof(int) * 2 * nrun);
   if (ce == cudaSuccess) ce = cudaMalloc(&e->d_err, sizeof(int));
-  if (ce == cudaSuccess) ce = cudaMemcpy(e->d_xneed, xneed.data(), sizeof(int) * nrun, cudaMemcpyHostToDevice);
+  if (ce == cudaSuccess) ce = cudaMemcpy(e->d_xneed, xneed.data(), sizeof(int) * 2 * nrun, cudaMemcpyHostToDevice);
   if (ce == cudaSuccess) ce = cudaMemset(e->d_err, 0, sizeof(int));
   if (ce != cudaSuccess) {
     ens_free(e);
     return fail(ce == cudaErrorMemoryAllocation ? SF_ENOMEM : SF_ECUDA, std::string("ensemble: ") + cudaGetErrorString(ce));
   }
   e->h_args.resize((size_t)6 * nrun);
-  e->blocks = ensemble_stage_blocks(std::max(e->xsmem, e->zsmem));
   *out = e;
   return SF_OK;
 }
@@ -1088,18 +1118,25 @@ int sf_ensemble_step(sf_ensemble* e, int nsteps) {
   }
   // the stage arguments of every member for both parities (h, factors and
   // pointers may have changed since the last call); the graphs read them
-  // from the device table
+  // from the device table, which is written when they did
+  bool changed = !e->args_set;
   for (int p = 0; p < 2; p++)
     for (int k = 0; k < 3; k++) {
       const int cur = (k == 1) ? 1 - p : p;
       for (int r = 0; r < R; r++) {
-        StageArgs a = stage_args(e->members[r], k, cur, false);
-        a.xslabs = 1;
-        e->h_args[((size_t)p * 3 + k) * R + r] = a;
+        StageArgs a;
+        std::memset(&a, 0, sizeof(a));   // the padding too: the copies are compared as bytes
+        a = stage_args(e->members[r], k, cur, false);
+        StageArgs& h = e->h_args[((size_t)p * 3 + k) * R + r];
+        changed = changed || std::memcmp(&h, &a, sizeof(a)) != 0;
+        std::memcpy(&h, &a, sizeof(a));
       }
     }
-  CK(cudaMemcpyAsync(e->d_args, e->h_args.data(), sizeof(StageArgs) * e->h_args.size(), cudaMemcpyHostToDevice,
-                     e->st));
+  if (changed) {
+    CK(cudaMemcpyAsync(e->d_args, e->h_args.data(), sizeof(StageArgs) * e->h_args.size(), cudaMemcpyHostToDevice,
+                       e->st));
+    e->args_set = true;
+  }
   for (int p = 0; p < 2; p++) {
     if (e->graph[p]) continue;
     cudaGraph_t gr;
@@ -1108,7 +1145,7 @@ int sf_ensemble_step(sf_ensemble* e, int nsteps) {
     for (int k = 0; k < 3; k++) {
       const StageArgs* a = e->d_args + ((size_t)p * 3 + k) * R;
       launch_ens_stage(a, e->d_x, e->nx, e->d_z, e->nz, e->d_counters + (size_t)k * (R + 1), e->d_xneed, e->d_err,
-                       e->blocks, std::max(e->xsmem, e->zsmem), e->st);
+                       e->blocks, e->smem, e->st);
     }
     cudaError_t ce = cudaStreamEndCapture(e->st, &gr);
     if (ce != cudaSuccess) return fail(SF_ECUDA, std::string("ensemble graph capture: ") + cudaGetErrorString(ce));
@@ -1141,9 +1178,12 @@ int sf_ensemble_profile(sf_ensemble* e, int nsteps, double* ms_x, double* ms_z) 
     CK(cudaEventRecord(ev[0], e->st));
     for (int k = 0; k < 3; k++) {
       const StageArgs* a = e->d_args + ((size_t)cur * 3 + k) * R;
-      launch_xpass_ens(a, e->d_x, e->nx, e->xsmem, e->st);
+      // the x items alone, then the z items alone (which then wait for none)
+      CK(cudaMemsetAsync(e->d_counters, 0, sizeof(int) * 3 * (R + 1), e->st));
+      launch_ens_stage(a, e->d_x, e->nx, e->d_z, 0, e->d_counters, e->d_xneed, e->d_err, e->blocks, e->smem, e->st);
       CK(cudaEventRecord(ev[1 + 2 * k], e->st));
-      launch_zstep_ens(a, e->d_z, e->nz, e->zsmem, e->st);
+      launch_ens_stage(a, e->d_x, 0, e->d_z, e->nz, e->d_counters + (R + 1), e->d_xneed + R, e->d_err, e->blocks,
+                       e->smem, e->st);
       CK(cudaEventRecord(ev[2 + 2 * k], e->st));
     }
     CK(cudaEventSynchronize(ev[6]));

@@ -15,6 +15,7 @@ pytestmark = pytest.mark.gpu
 
 # mode, N1, N2, N3, runs
 CASES = [
+    ("nonlinear", 16, 1, 260, 64), ("linear", 16, 1, 36, 2),
     ("nonlinear", 32, 1, 256, 33), ("nonlinear", 64, 1, 100, 41), ("nonlinear", 128, 1, 132, 16),
     ("nonlinear", 256, 1, 260, 4), ("nonlinear", 512, 1, 132, 4), ("nonlinear", 64, 16, 36, 2),
     ("linear", 32, 1, 36, 1), ("linear", 64, 1, 44, 3), ("linear", 128, 1, 68, 1), ("linear", 256, 1, 36, 2),
