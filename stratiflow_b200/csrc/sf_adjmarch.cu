@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(AMShape<N1, D3>::WARPS * 32, 1) k_adjmarch(con
   float4* dring = ring + 2 * N1;                    // U1T, BT, U3T, U2T
   float4* tbuf = dring + 2 * N1;
   float4* cbuf = tbuf + T::TB;                      // [2][NKS][G]: (c1, cB), (c2, c3) awaiting their z terms
-  float2* stg = reinterpret_cast<float2*>(cbuf + 2 * NKS * G);   // [ROWS][K1]
+  float2* stg = reinterpret_cast<float2*>(cbuf + 2 * NKS * G);   // 3D [6][K1] pairs, 2D [6][K1]
   __syncthreads();
   const int partner_lane = (lane & ~(G - 1)) | ((G - l) & (G - 1));
   float4 w1[8];
@@ -107,29 +107,39 @@ __global__ void __launch_bounds__(AMShape<N1, D3>::WARPS * 32, 1) k_adjmarch(con
     }
     const float Ri = a.Ri[run];
     const size_t tstride = D3 ? (size_t)N2 * K1 : (size_t)g.Pp, fstride = (size_t)N3 * tstride;
-    float2* __restrict__ dst = D3 ? a.mixout + (size_t)run * 8 * fstride + (size_t)y * K1 : a.rnl + (size_t)run * 4 * fstride;
+    float2* __restrict__ dst = D3 ? a.mixout + 2 * ((size_t)run * 4 * fstride + (size_t)y * K1) : a.rnl + (size_t)run * 4 * fstride;
     const float2* __restrict__ mean = a.adir + (size_t)run * 4 * N3 * g.Pp;   // (0,0) modes of the direct totals
 
-    // the input rows of level t: adjoint u1, u3, b, (u2); direct; (their y derivatives)
+    // the input rows of level t: the adjoint fields, the direct ones, (their y
+    // derivatives); 3D as the pairs (u1, u3), (b, u2), 2D as rows u1, u3, b
     auto prefetch = [&](int t) {
       if (t < 0 || t >= N3) return;
 #pragma unroll
-      for (int i = 0; i < ROWS; i++) {
-        const int r = i % H, f = r == 0 ? 0 : (r == 1 ? 2 : (r == 2 ? 3 : 1));
-        const float2* src = D3 ? a.amix + (size_t)(run * 12 + 4 * (i / H) + f) * fstride + (size_t)y * K1
-                               : (i < H ? a.S + (size_t)(run * 5 + f) * fstride : a.adir + (size_t)(run * 4 + f) * fstride);
-        src += (size_t)t * tstride + l;
+      for (int i = 0; i < 6; i++) {
+        if (D3) {
+          const float2* src = a.amix + 2 * ((size_t)(run * 6 + i) * fstride + (size_t)y * K1 + (size_t)t * tstride + l);
 #pragma unroll
-        for (int j = 0; j < (K1 + G - 1) / G; j++)
-          if (l + G * j < K1) xm_cp8(stg + i * K1 + l + G * j, src + G * j);
+          for (int j = 0; j < (K1 + G - 1) / G; j++)
+            if (l + G * j < K1) xm_cp16(stg + 2 * (i * K1 + l + G * j), src + 2 * G * j);
+        } else {
+          const int r = i % 3, f = r == 0 ? 0 : r + 1;
+          const float2* src = (i < 3 ? a.S + (size_t)(run * 5 + f) * fstride : a.adir + (size_t)(run * 4 + f) * fstride);
+          src += (size_t)t * tstride + l;
+#pragma unroll
+          for (int j = 0; j < (K1 + G - 1) / G; j++)
+            if (l + G * j < K1) xm_cp8(stg + i * K1 + l + G * j, src + G * j);
+        }
       }
     };
     auto kk = [&](int i) { return T::kmode(l, i); };
     auto Ca = [&](int i) -> float4& { return cbuf[i * G + l]; };
     auto Cb = [&](int i) -> float4& { return cbuf[(NKS + i) * G + l]; };
-    auto store = [&](int c, int lvl, int i, float2 v) {
-      const int cc = D3 ? c : (c == 0 ? 0 : (c == 4 ? 2 : 3));
-      if (D3 || (lvl >= 0 && lvl < N3)) dst[(size_t)cc * fstride + (size_t)lvl * tstride + kk(i)] = v;
+    // 3D: the pair p of combinations; 2D: field f (r1, r3, rB) alone
+    auto store2 = [&](int p, int lvl, int i, float2 v, float2 w) {
+      reinterpret_cast<float4*>(dst)[(size_t)p * fstride + (size_t)lvl * tstride + kk(i)] = make_float4(v.x, v.y, w.x, w.y);
+    };
+    auto store = [&](int f, int lvl, int i, float2 v) {
+      if (lvl >= 0 && lvl < N3) dst[(size_t)f * fstride + (size_t)lvl * tstride + kk(i)] = v;
     };
     auto ikx = [&](float k, float2 v) { return make_float2(-k * v.y, k * v.x); };
 
@@ -150,9 +160,8 @@ __global__ void __launch_bounds__(AMShape<N1, D3>::WARPS * 32, 1) k_adjmarch(con
       const bool lv = t >= 0 && t < N3, lvm = tm >= 0 && tm < N3;
       float4 *cur = ring + (size_t)(k & 1) * N1, *dcur = dring + (size_t)(k & 1) * N1;
       const float4 *prev = ring + (size_t)((k - 1) & 1) * N1, *dprev = dring + (size_t)((k - 1) & 1) * N1;
-      // the c2r input of the pair (row 0 + i row 1, row 2 + i row 3) of st, times i kx with DX
-      auto rows = [&](c2x (&x)[E], const float2* st, bool has4, bool DX) {
-        const float2 *r0 = st, *r1 = st + K1, *r2 = st + 2 * K1, *r3 = st + 3 * K1;
+      // the c2r input of the pair (u1 + i u3, b + i u2) of the rows at st, times i kx with DX
+      auto rows = [&](c2x (&x)[E], const float2* st, bool DX) {
 #pragma unroll
         for (int e = 0; e < E; e++) {
           x[e] = c2x{make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
@@ -163,7 +172,18 @@ __global__ void __launch_bounds__(AMShape<N1, D3>::WARPS * 32, 1) k_adjmarch(con
           const float on = (dir || cnj) ? 1.f : 0.f;
           const float sg = dir ? -1.f : 1.f;
           const float im0 = (n == 0) ? 0.f : on;             // k = 0: real parts only
-          float2 A = r0[m], B = r1[m], C_ = r2[m], D = has4 ? r3[m] : make_float2(0.f, 0.f);
+          float2 A, B, C_, D = make_float2(0.f, 0.f);
+          if (D3) {
+            const float4 p = reinterpret_cast<const float4*>(st)[m], q = reinterpret_cast<const float4*>(st)[K1 + m];
+            A = make_float2(p.x, p.y);
+            B = make_float2(p.z, p.w);
+            C_ = make_float2(q.x, q.y);
+            D = make_float2(q.z, q.w);
+          } else {
+            A = st[m];
+            B = st[K1 + m];
+            C_ = st[2 * K1 + m];
+          }
           if (DX) {
             const float kx = __ldg(a.kx + m0);
             A = ikx(kx, A);
@@ -180,7 +200,7 @@ __global__ void __launch_bounds__(AMShape<N1, D3>::WARPS * 32, 1) k_adjmarch(con
       __syncwarp();
       {
         c2x x[E];
-        rows(x, stg, D3, false);
+        rows(x, stg, false);
         T::template fft<true>(x, tbuf, tw4, tw2, l, w1);
 #pragma unroll
         for (int s = 0; s < E; s++) cur[s * G + l] = c2x_f4(x[s]);
@@ -188,7 +208,7 @@ __global__ void __launch_bounds__(AMShape<N1, D3>::WARPS * 32, 1) k_adjmarch(con
       }
       {
         c2x x[E];
-        rows(x, stg + H * K1, D3, false);
+        rows(x, stg + H * K1, false);
         T::template fft<true>(x, tbuf, tw4, tw2, l, w1);
 #pragma unroll
         for (int s = 0; s < E; s++) dcur[s * G + l] = c2x_f4(x[s]);
@@ -214,7 +234,7 @@ __global__ void __launch_bounds__(AMShape<N1, D3>::WARPS * 32, 1) k_adjmarch(con
       };
       {
         c2x x[E];
-        rows(x, stg + H * K1, D3, true);
+        rows(x, stg + H * K1, true);
         if (!D3) {
           __syncwarp();   // the staged rows are read: the next level's copies may start
           if (k <= n) prefetch(t + 1);
@@ -225,7 +245,7 @@ __global__ void __launch_bounds__(AMShape<N1, D3>::WARPS * 32, 1) k_adjmarch(con
       }
       if constexpr (D3) {
         c2x x[E];
-        rows(x, stg + 2 * H * K1, true, false);
+        rows(x, stg + 2 * H * K1, false);
         __syncwarp();
         if (k <= n) prefetch(t + 1);
         T::template fft<true>(x, tbuf, tw4, tw2, l, w1);
@@ -321,10 +341,17 @@ __global__ void __launch_bounds__(AMShape<N1, D3>::WARPS * 32, 1) k_adjmarch(con
             const float2 Dp = D3 ? B2 : B1;
             if (fin) {
               const float4 ca = Ca(i), cb = Cb(i);
-              store(0, tm, i, make_float2(ca.x + fu * A1.x, ca.y + fu * A1.y));
-              store(6, tm, i, make_float2(ca.z + fu * A2.x, ca.w + fu * A2.y));
-              if (D3) store(2, tm, i, make_float2(cb.x + fu * B1.x, cb.y + fu * B1.y));
-              store(4, tm, i, make_float2(cb.z + fd * Dp.x, cb.w + fd * Dp.y));
+              const float2 c1 = make_float2(ca.x + fu * A1.x, ca.y + fu * A1.y);
+              const float2 cB = make_float2(ca.z + fu * A2.x, ca.w + fu * A2.y);
+              const float2 c3 = make_float2(cb.z + fd * Dp.x, cb.w + fd * Dp.y);
+              if (D3) {
+                store2(0, tm, i, c1, cB);
+                store2(2, tm, i, make_float2(cb.x + fu * B1.x, cb.y + fu * B1.y), c3);
+              } else {
+                store(0, tm, i, c1);
+                store(2, tm, i, c3);
+                store(3, tm, i, cB);
+              }
             }
             Ca(i) = make_float4(sd * A1.x, sd * A1.y, sd * A2.x, sd * A2.y);
             Cb(i) = D3 ? make_float4(sd * B1.x, sd * B1.y, ndl * Dp.x, ndl * Dp.y)
@@ -337,10 +364,8 @@ __global__ void __launch_bounds__(AMShape<N1, D3>::WARPS * 32, 1) k_adjmarch(con
             Cb(i) = D3 ? make_float4(cb.x + b1.x, cb.y + b1.y, cb.z + b2.x, cb.w + b2.y)
                        : make_float4(0.f, 0.f, cb.z + b1.x, cb.w + b1.y);
           } else {   // U1 U2T, U2 U2T, Tilde(U2T) U3, B U2T
-            store(1, t, i, A1);
-            store(3, t, i, A2);
-            store(5, t, i, B1);
-            store(7, t, i, B2);
+            store2(1, t, i, A1, B2);
+            store2(3, t, i, A2, B1);
           }
         }
         tok = __float_as_int(z[0].re.x) & rz;

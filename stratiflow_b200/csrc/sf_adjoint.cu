@@ -21,7 +21,7 @@
 
 #include <algorithm>
 
-#include "sf_fft.cuh"
+#include "sf_fft2.cuh"
 #include "sf_internal.cuh"
 
 namespace sf {
@@ -312,41 +312,56 @@ __global__ void __launch_bounds__(kAdjGroups * 32) k_xpass_adj(StageArgs a, int 
 }
 
 // ---------------------------------------------------------------- 3D ----
-// The 12 fields of the 3D adjoint x pass, inverse-transformed along y:
-// the adjoint u1, u2, u3, b; the direct totals u1T, u2T, u3T, bT; and ddy of
-// the direct totals (i ky applied on the modal rows). [nrun][12][N3][N2][K1]
+// The 12 fields of the 3D adjoint x pass, inverse-transformed along y in
+// packed pairs (u1, u3), (b, u2): of the adjoint; of the direct totals; of ddy
+// of the direct totals (i ky applied on the modal rows).
+// [nrun][6][N3][N2][K1][2], blockIdx.z = 6 run + pair
 constexpr int kYT = 128;
 template <int N2>
 __host__ __device__ constexpr int ycols_adj() { return (kYT / 32) * (32 / FFTShape<N2>::G); }
 
 template <int N2>
 __global__ void __launch_bounds__(kYT) k_ifft_y_adj(StageArgs a) {
-  constexpr int G = FFTShape<N2>::G, E = FFTShape<N2>::E, BUF = fft_buf_stride<N2>();
+  using Y = YT2<N2>;
+  constexpr int G = Y::G, E = Y::E;
   const Geo g = a.g;
-  __shared__ float2 fbuf[(kYT / G) * BUF];
+  __shared__ float4 fbuf4[(kYT / G) * Y::BUF];
+  __shared__ float4 tw4[Y::TWE];
+  __shared__ __align__(16) float2 tw2[Y::TWE];
   const int grp = threadIdx.x / G, l = threadIdx.x % G;
   const int j1 = blockIdx.x * ycols_adj<N2>() + grp;
   const int j = blockIdx.y;
-  const int run = blockIdx.z / 12, f = blockIdx.z % 12;
+  const int run = blockIdx.z / 6, p = blockIdx.z % 6;
   const bool act = j1 < g.K1;
-  const float2* src = f < 4 ? a.S + ((size_t)(run * 5 + f) * g.N3 + j) * g.Pp
-                            : a.adir + ((size_t)(run * 4 + (f & 3)) * g.N3 + j) * g.Pp;
-  float2 x[E];
+  const int fA = (p & 1) ? 3 : 0, fB = (p & 1) ? 1 : 2;
+  const float2* base = p < 2 ? a.S + (size_t)run * 5 * g.fblk : a.adir + (size_t)run * 4 * g.fblk;
+  const float2 *srcA = base + ((size_t)fA * g.N3 + j) * g.Pp + j1, *srcB = base + ((size_t)fB * g.N3 + j) * g.Pp + j1;
+  c2x x[E];
 #pragma unroll
   for (int e = 0; e < E; e++) {
     const int n2 = l + G * e;
     int q = -1;
     if (n2 < g.Ky) q = n2;
     else if (n2 > N2 - g.Ky) q = n2 - (N2 - g.K2);
-    float2 v = (act && q >= 0) ? src[q * g.K1 + j1] : make_float2(0.f, 0.f);
-    if (f >= 8 && q >= 0) v = cik(a.ky[q], v);
-    x[e] = v;
+    float2 A = make_float2(0.f, 0.f), B = A;
+    if (act && q >= 0) {
+      A = srcA[(size_t)q * g.K1];
+      B = srcB[(size_t)q * g.K1];
+      if (p >= 4) {
+        A = cik(a.ky[q], A);
+        B = cik(a.ky[q], B);
+      }
+    }
+    x[e] = c2x{make_float2(A.x, B.x), make_float2(A.y, B.y)};
   }
-  reg_fft<N2, true>(x, fbuf + grp * BUF, a.tw, l);
+  Y::fill(tw4, tw2, a.tw, threadIdx.x, kYT);
+  __syncthreads();
+  Y::template fft<true>(x, fbuf4 + grp * Y::BUF, tw4, tw2, l);
   if (act) {
-    float2* dst = a.amix + ((size_t)(run * 12 + f) * g.N3 + j) * N2 * g.K1 + j1;
+    float4* dst = reinterpret_cast<float4*>(a.amix) + ((size_t)(run * 6 + p) * g.N3 + j) * N2 * g.K1 + j1;
 #pragma unroll
-    for (int sl = 0; sl < E; sl++) dst[(size_t)reg_fft_out_index<N2>(l, sl) * g.K1] = x[sl];
+    for (int sl = 0; sl < E; sl++)
+      dst[(size_t)Y::out(l, sl) * g.K1] = make_float4(x[sl].re.x, x[sl].im.x, x[sl].re.y, x[sl].im.y);
   }
 }
 
@@ -413,7 +428,8 @@ __global__ void __launch_bounds__(kAdj3Groups * FFTShape<N1>::G) k_xpass_adj3(St
   for (int i = threadIdx.x; i < 12 * NS * K1; i += blockDim.x) {
     const int fb = i / (NS * K1), r = i - fb * NS * K1, s = r / K1, k = r - s * K1;
     const int t = j0 - 1 + s;
-    stg[i] = (t >= 0 && t < N3) ? a.amix[(((size_t)(run * 12 + fb) * N3 + t) * g.N2 + y) * K1 + k]
+    const int f = fb & 3;
+    stg[i] = (t >= 0 && t < N3) ? a.amix[mix_pair(g, run * 6 + 2 * (fb >> 2), mix_in_pair(f), mix_in_side(f), t, y) + 2 * k]
                                 : make_float2(0.f, 0.f);
   }
   for (int s = threadIdx.x; s < NS; s += blockDim.x) {   // HorizontalAverage: the (0,0) modes
@@ -582,16 +598,15 @@ __global__ void __launch_bounds__(kAdj3Groups * FFTShape<N1>::G) k_xpass_adj3(St
     if (t >= 2)
       dnd = cadd(cscale(H(A_DU3DU3T, s - 1, k), zc[ZC_DND_LO * N3 + t]),
                  cscale(H(A_DU3DU3T, s, k), zc[ZC_DND_DI * N3 + t]));
-    float2* m = a.mixout + (((size_t)run * 8 * N3 + t) * g.N2 + y) * K1 + k;
+    float4* m = reinterpret_cast<float4*>(a.mixout) + (((size_t)run * 4 * N3 + t) * g.N2 + y) * K1 + k;
+    auto pair = [](float2 v, float2 w) { return make_float4(v.x, v.y, w.x, w.y); };
     const size_t cs = g.mblk;
-    m[0 * cs] = cadd(cadd(cik(kxv, H(A_U1U1T, s, k)), dzdn(A_BU1_U3T)), H(A_F1, s, k));
-    m[1 * cs] = H(A_U1U2T, s, k);
-    m[2 * cs] = cadd(cadd(cik(kxv, H(A_U2U1T, s, k)), dzdn(A_BU2_U3T)), H(A_F2, s, k));
-    m[3 * cs] = H(A_U2U2T, s, k);
-    m[4 * cs] = cadd(cadd(cik(kxv, H(A_TU1T_U3, s, k)), dnd), H(A_F3, s, k));
-    m[5 * cs] = H(A_TU2T_U3, s, k);
-    m[6 * cs] = cadd(cadd(dzdn(A_BB_U3T), cik(kxv, H(A_BU1T, s, k))), H(A_FB, s, k));
-    m[7 * cs] = H(A_BU2T, s, k);
+    m[0 * cs] = pair(cadd(cadd(cik(kxv, H(A_U1U1T, s, k)), dzdn(A_BU1_U3T)), H(A_F1, s, k)),
+                     cadd(cadd(dzdn(A_BB_U3T), cik(kxv, H(A_BU1T, s, k))), H(A_FB, s, k)));
+    m[1 * cs] = pair(H(A_U1U2T, s, k), H(A_BU2T, s, k));
+    m[2 * cs] = pair(cadd(cadd(cik(kxv, H(A_U2U1T, s, k)), dzdn(A_BU2_U3T)), H(A_F2, s, k)),
+                     cadd(cadd(cik(kxv, H(A_TU1T_U3, s, k)), dnd), H(A_F3, s, k)));
+    m[3 * cs] = pair(H(A_U2U2T, s, k), H(A_TU2T_U3, s, k));
   }
 }
 
@@ -607,7 +622,7 @@ void adj3_launch(const StageArgs& a, cudaStream_t st) {
 
 template <int N2>
 void ify_adj_launch(const StageArgs& a, cudaStream_t st) {
-  k_ifft_y_adj<N2><<<dim3(adiv(a.g.K1, ycols_adj<N2>()), a.g.N3, a.g.nrun * 12), kYT, 0, st>>>(a);
+  k_ifft_y_adj<N2><<<dim3(adiv(a.g.K1, ycols_adj<N2>()), a.g.N3, a.g.nrun * 6), kYT, 0, st>>>(a);
 }
 
 template <int N1>

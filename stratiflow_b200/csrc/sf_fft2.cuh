@@ -263,12 +263,12 @@ __device__ __forceinline__ void fill_tw2_128h(float4* tw4, float2* tw2, const fl
     t2[i] = make_float4(w.x, w.x, w.y, w.y);
   }
 }
-template <bool INV>
-__device__ __forceinline__ void reg_fft2_128h(c2x (&x)[8], float4* buf, const float2* __restrict__ tw2, int l,
-                                              const float4 (&w1)[8]) {
+template <bool INV, class TW1>
+__device__ __forceinline__ void reg_fft2_128h_body(c2x (&x)[8], float4* buf, const float2* __restrict__ tw2, int l,
+                                                   const TW1& twid) {
   dft2<8, INV>(x);
 #pragma unroll
-  for (int k1 = 1; k1 < 8; k1++) x[k1] = tw2_mul_reg<INV>(x[k1], w1[k1]);
+  for (int k1 = 1; k1 < 8; k1++) twid(x[k1], k1);
   __syncwarp();
 #pragma unroll
   for (int k1 = 0; k1 < 8; k1++) buf[k1 * 17 + l] = c2x_to4(x[k1]);    // element (row l, column k1)
@@ -297,6 +297,52 @@ __device__ __forceinline__ void reg_fft2_128h(c2x (&x)[8], float4* buf, const fl
 #pragma unroll
   for (int i = 0; i < 2; i++) dft2<4, INV>(x + 4 * i);
 }
+
+// first-stage twiddles from registers (a kernel of many transforms), or from the table
+template <bool INV>
+__device__ __forceinline__ void reg_fft2_128h(c2x (&x)[8], float4* buf, const float2* __restrict__ tw2, int l,
+                                              const float4 (&w1)[8]) {
+  reg_fft2_128h_body<INV>(x, buf, tw2, l, [&](c2x& v, int k1) { v = tw2_mul_reg<INV>(v, w1[k1]); });
+}
+template <bool INV>
+__device__ __forceinline__ void reg_fft2_128h(c2x (&x)[8], float4* buf, const float4* __restrict__ tw4,
+                                              const float2* __restrict__ tw2, int l) {
+  reg_fft2_128h_body<INV>(x, buf, tw2, l, [&](c2x& v, int k1) { tw2_apply<INV>(v, tw4 + k1 * 16 + l, tw2); });
+}
+
+// The lane layout of a y transform pair: G lanes per column, E points per lane
+// (in[l + G e] in slot e), out(l, s) the output index in slot s. YT2: the
+// two-stage transform over FFTShape's lanes. YT: the same, but 16 lanes of 8
+// points for N = 128: with 16 points a lane, the two pairs that k_fft_y holds
+// need 186 registers and leave 8 warps per SM, too few loads in flight
+// (256x128x384: 123 us against 115; k_ifft_y2, which holds one pair, is the
+// faster with four columns a warp, 56 against 64).
+template <int N>
+struct YT2 {
+  static constexpr int G = FFTShape<N>::G, E = FFTShape<N>::E, TWE = E * G, BUF = fft2_buf_elems<N>();
+  __device__ __forceinline__ static int out(int l, int s) { return reg_fft_out_index<N>(l, s); }
+  __device__ __forceinline__ static void fill(float4* tw4, float2* tw2, const float2* tw, int tid, int nthr) {
+    fill_tw2<N>(tw4, tw2, tw, tid, nthr);
+  }
+  template <bool INV>
+  __device__ __forceinline__ static void fft(c2x (&x)[E], float4* buf, const float4* tw4, const float2* tw2, int l) {
+    reg_fft2<N, INV>(x, buf, tw4, tw2, l);
+  }
+};
+template <int N>
+struct YT : YT2<N> {};
+template <>
+struct YT<128> {
+  static constexpr int G = 16, E = 8, TWE = 128, BUF = 8 * 17;
+  __device__ __forceinline__ static int out(int l, int s) { return l + 16 * (s / 4 + 2 * (s % 4)); }
+  __device__ __forceinline__ static void fill(float4* tw4, float2* tw2, const float2* tw, int tid, int nthr) {
+    fill_tw2_128h(tw4, tw2, tw, tid, nthr);
+  }
+  template <bool INV>
+  __device__ __forceinline__ static void fft(c2x (&x)[E], float4* buf, const float4* tw4, const float2* tw2, int l) {
+    reg_fft2_128h<INV>(x, buf, tw4, tw2, l);
+  }
+};
 
 // The packed transform pair of N = 512 points over a whole warp (32 lanes,
 // 16 points each): as reg_fft2_256w with 16 columns k1: a 16-point DFT over e

@@ -7,8 +7,10 @@
 //                                       stage (the zeta term of ExplicitRK)
 //   rnl             [nrun][4][N3][Pp]   nonlinear terms of this stage
 //   qbuf            [nrun][N3][Pp]      forward-sweep scratch of the pressure solve
-//   mixin  (3D)     [nrun][4][N3][N2][K1]  fields after the inverse y transform
-//   mixout (3D)     [nrun][8][N3][N2][K1]  x-transformed product combinations
+//   mixin  (3D)     [nrun][2][N3][N2][K1][2]  fields after the inverse y
+//                   transform, two side by side: (u1, u3), (b, u2)
+//   mixout (3D)     [nrun][4][N3][N2][K1][2]  x-transformed product
+//                   combinations: (C_1, C_B), (C_1y, C_By), (C_2, C_3), (C_2y, C_3y)
 //   base            [nrun][4][N3][N2][N1]  frozen nodal base of the linear step
 // Pp = roundup(K1*K2, 16) is the plane stride of one level; mode m = q*K1+j1.
 #pragma once
@@ -79,7 +81,7 @@ struct StageArgs {
   int xslabs;       // slabs per x-pass block (0: chosen by the launcher)
   int adjoint;      // adjoint step: no linear buoyancy terms in the z solve
   const float2* adir;   // adjoint step: the direct total state of the substep [nrun][4][N3][Pp]
-  float2* amix;         // 3D adjoint step: 12 y-transformed fields [nrun][12][N3][N2][K1]
+  float2* amix;         // 3D adjoint step: 12 y-transformed fields [nrun][6][N3][N2][K1][2], paired as mixin
   float adj_invK;       // adjoint step: 1/K of the mixing objective (IMEXRK.h:487)
   float h, hz, hb, cv, cb, pm;
   // level band of one launch of the y transforms (levels lvl0 .. lvl0+nlvl-1;
@@ -192,6 +194,13 @@ int launch_base_nodal(const Geo& g, const float2* kept_modal, int field, float* 
 
 // ------------------------------------------------------- device helpers ----
 #ifdef __CUDACC__
+// where field f of mixin's pairs lies, and the first element of row (t, y) of
+// pair p after pair0, on its side
+__device__ __forceinline__ int mix_in_pair(int f) { return f == 0 || f == 2 ? 0 : 1; }
+__device__ __forceinline__ int mix_in_side(int f) { return f == 2 || f == 1 ? 1 : 0; }
+__device__ __forceinline__ size_t mix_pair(const Geo& g, int pair0, int p, int side, int t, int y) {
+  return ((((size_t)(pair0 + p) * g.N3 + t) * g.N2 + y) * g.K1) * 2 + side;
+}
 __device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {

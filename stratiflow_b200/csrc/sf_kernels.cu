@@ -34,9 +34,14 @@ __device__ __forceinline__ int n2_of_q(int q, int Ky, int K2, int N2) { return q
 template <int N2>
 __host__ __device__ constexpr int ycols() { return (kYThreads / 32) * (32 / FFTShape<N2>::G); }
 
-// modal [q][j1] of (run, field f, level j) -> mixed [y][j1], inverse c2c in y.
-// One lane group per kx column; consecutive columns in consecutive groups so
-// that a warp's loads of one y row cover whole 32-byte sectors.
+// the same in the pair kernels
+template <int N2>
+__host__ __device__ constexpr int ypcols() { return (kYThreads / 32) * (32 / YT<N2>::G); }
+
+// modal [q][j1] of (run, field f, level j) -> plain rows [y][j1] of that field,
+// inverse c2c in y (the nodal fields of files, bases and diagnostics). One lane
+// group per kx column; consecutive columns in consecutive groups so that a
+// warp's loads of one y row cover whole 32-byte sectors.
 template <int N2>
 __global__ void __launch_bounds__(kYThreads, 8) k_ifft_y(StageArgs a) {
   constexpr int G = FFTShape<N2>::G, E = FFTShape<N2>::E, BUF = fft_buf_stride<N2>();
@@ -67,25 +72,28 @@ __global__ void __launch_bounds__(kYThreads, 8) k_ifft_y(StageArgs a) {
   }
 }
 
-// The same for fields (2p, 2p+1) of every run at once (blockIdx.z = 2 run +
-// p): each lane group transforms its column of both fields as one packed pair
-// of transforms (sf_fft2.cuh), half the FP32 instructions of two transforms.
+// The same for the field pairs of every run (blockIdx.z = 2 run + p; p = 0
+// (u1, u3), p = 1 (b, u2)): each lane group transforms its column of both
+// fields as one packed pair of transforms (sf_fft2.cuh), half the FP32
+// instructions of two transforms, and stores them side by side, one 16-byte
+// value per mode: four columns of a warp are 64 contiguous bytes of a row, not
+// 32 of two rows. Bound by DRAM and by the L1's requests; 256x128x384: YIA
+// us with the fields apart, now YIB.
 template <int N2>
 __global__ void __launch_bounds__(kYThreads) k_ifft_y2(StageArgs a) {
-  constexpr int G = FFTShape<N2>::G, E = FFTShape<N2>::E;
+  using Y = YT2<N2>;
+  constexpr int G = Y::G, E = Y::E;
   const Geo g = a.g;
-  __shared__ float4 fbuf4[(kYThreads / G) * fft2_buf_elems<N2>()];
-  __shared__ float4 tw4[E * G];
-  __shared__ float2 tw2[E * G];
-  fill_tw2<N2>(tw4, tw2, a.tw, threadIdx.x, kYThreads);
-  __syncthreads();
+  __shared__ float4 fbuf4[(kYThreads / G) * Y::BUF];
+  __shared__ float4 tw4[Y::TWE];
+  __shared__ __align__(16) float2 tw2[Y::TWE];
   const int grp = threadIdx.x / G, l = threadIdx.x % G;
   const int j1 = blockIdx.x * ycols<N2>() + grp;
   const int j = blockIdx.y + a.lvl0;
-  const int run = blockIdx.z >> 1, f0 = 2 * (blockIdx.z & 1);
+  const int run = blockIdx.z >> 1, p = blockIdx.z & 1;
   const bool act = j1 < g.K1;
-  const float2* srcA = a.S + ((size_t)(run * 5 + f0) * g.N3 + j) * g.Pp + j1;
-  const float2* srcB = srcA + (size_t)g.N3 * g.Pp;
+  const float2* srcA = a.S + ((size_t)(run * 5 + (p ? 3 : 0)) * g.N3 + j) * g.Pp + j1;
+  const float2* srcB = a.S + ((size_t)(run * 5 + (p ? 1 : 2)) * g.N3 + j) * g.Pp + j1;
   c2x x[E];
 #pragma unroll
   for (int e = 0; e < E; e++) {
@@ -98,56 +106,67 @@ __global__ void __launch_bounds__(kYThreads) k_ifft_y2(StageArgs a) {
     const float2 B = in ? srcB[(size_t)q * g.K1] : make_float2(0.f, 0.f);
     x[e] = c2x{make_float2(A.x, B.x), make_float2(A.y, B.y)};
   }
-  reg_fft2<N2, true>(x, fbuf4 + grp * fft2_buf_elems<N2>(), tw4, tw2, l);
+  // the tables after this block's loads are on their way
+  Y::fill(tw4, tw2, a.tw, threadIdx.x, kYThreads);
+  __syncthreads();
+  Y::template fft<true>(x, fbuf4 + grp * Y::BUF, tw4, tw2, l);
   if (act) {
-    float2* dA = a.mixin + ((size_t)(run * 4 + f0) * g.N3 + j) * N2 * g.K1 + j1;
-    float2* dB = dA + (size_t)g.N3 * N2 * g.K1;
+    float4* dst = reinterpret_cast<float4*>(a.mixin) + ((size_t)(run * 2 + p) * g.N3 + j) * N2 * g.K1 + j1;
 #pragma unroll
-    for (int sl = 0; sl < E; sl++) {
-      const size_t o = (size_t)reg_fft_out_index<N2>(l, sl) * g.K1;
-      dA[o] = make_float2(x[sl].re.x, x[sl].im.x);
-      dB[o] = make_float2(x[sl].re.y, x[sl].im.y);
-    }
+    for (int sl = 0; sl < E; sl++)
+      dst[(size_t)Y::out(l, sl) * g.K1] = make_float4(x[sl].re.x, x[sl].im.x, x[sl].re.y, x[sl].im.y);
   }
 }
 
-// mixed combos (C_f, C_fy) [y][j1] -> r_f[q][j1] = Fy(C_f) + i ky Fy(C_fy)
+// The combination pairs of two fields (blockIdx.z = 2 run + p; p = 0 the
+// fields 1 and B, p = 1 the fields 2 and 3): r_f[q][j1] = Fy(C_f) + i ky
+// Fy(C_fy). The pair of the C_fy is transformed first and waits, times i ky, in
+// the registers; both are read as one 16-byte value per mode and row (see
+// k_ifft_y2). 256x128x384: YFA us with every combination apart, now YFB.
 template <int N2>
 __global__ void __launch_bounds__(kYThreads) k_fft_y(StageArgs a) {
-  constexpr int G = FFTShape<N2>::G, E = FFTShape<N2>::E;
+  using Y = YT<N2>;
+  constexpr int G = Y::G, E = Y::E;
   const Geo g = a.g;
-  __shared__ float4 fbuf4[(kYThreads / G) * fft2_buf_elems<N2>()];
-  __shared__ float4 tw4[E * G];
-  __shared__ float2 tw2[E * G];
-  fill_tw2<N2>(tw4, tw2, a.tw, threadIdx.x, kYThreads);
-  __syncthreads();
+  __shared__ float4 fbuf4[(kYThreads / G) * Y::BUF];
+  __shared__ float4 tw4[Y::TWE];
+  __shared__ __align__(16) float2 tw2[Y::TWE];
   const int grp = threadIdx.x / G, l = threadIdx.x % G;
-  const int j1 = blockIdx.x * ycols<N2>() + grp;
+  const int j1 = blockIdx.x * ypcols<N2>() + grp;
   const int j = blockIdx.y + a.lvl0;
-  const int run = blockIdx.z >> 2, f = blockIdx.z & 3;
+  const int run = blockIdx.z >> 1, p = blockIdx.z & 1;
   const bool act = j1 < g.K1;
-  const float2* cA = a.mixout + ((size_t)(run * 8 + 2 * f) * g.N3 + j) * N2 * g.K1 + j1;
-  const float2* cB = a.mixout + ((size_t)(run * 8 + 2 * f + 1) * g.N3 + j) * N2 * g.K1 + j1;
-  // (C_f, C_fy) as one packed pair of transforms (sf_fft2.cuh)
-  c2x x[E];
+  const size_t ps = (size_t)g.N3 * N2 * g.K1;   // one pair's values
+  const float4* src = reinterpret_cast<const float4*>(a.mixout) + (size_t)(run * 4 + 2 * p) * ps + (size_t)j * N2 * g.K1 + j1;
+  float4* buf = fbuf4 + grp * Y::BUF;
+  c2x y[E], x[E];
 #pragma unroll
   for (int e = 0; e < E; e++) {
     const size_t o = (size_t)(l + G * e) * g.K1;
-    const float2 A = act ? cA[o] : make_float2(0.f, 0.f), B = act ? cB[o] : make_float2(0.f, 0.f);
-    x[e] = c2x{make_float2(A.x, B.x), make_float2(A.y, B.y)};
+    const float4 v = act ? __ldcs(src + ps + o) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 w = act ? __ldcs(src + o) : make_float4(0.f, 0.f, 0.f, 0.f);
+    y[e] = c2x{make_float2(v.x, v.z), make_float2(v.y, v.w)};
+    x[e] = c2x{make_float2(w.x, w.z), make_float2(w.y, w.w)};
   }
-  reg_fft2<N2, false>(x, fbuf4 + grp * fft2_buf_elems<N2>(), tw4, tw2, l);
+  // the tables after this block's loads are on their way
+  Y::fill(tw4, tw2, a.tw, threadIdx.x, kYThreads);
+  __syncthreads();
+  Y::template fft<false>(y, buf, tw4, tw2, l);
+  Y::template fft<false>(x, buf, tw4, tw2, l);
   if (act) {
-    float2* dst = a.rnl + ((size_t)(run * 4 + f) * g.N3 + j) * g.Pp + j1;
+    float2* dA = a.rnl + ((size_t)(run * 4 + (p ? 1 : 0)) * g.N3 + j) * g.Pp + j1;
+    float2* dB = a.rnl + ((size_t)(run * 4 + (p ? 2 : 3)) * g.N3 + j) * g.Pp + j1;
 #pragma unroll
     for (int sl = 0; sl < E; sl++) {
-      const int n2 = reg_fft_out_index<N2>(l, sl);
+      const int n2 = Y::out(l, sl);
       int q = -1;
       if (n2 < g.Ky) q = n2;
       else if (n2 > N2 - g.Ky) q = n2 - (N2 - g.K2);
-      if (q >= 0) {   // Fy(C_f) + i ky Fy(C_fy)
-        const float ky = a.ky[q];
-        dst[(size_t)q * g.K1] = make_float2(x[sl].re.x - ky * x[sl].im.y, x[sl].im.x + ky * x[sl].re.y);
+      if (q >= 0) {
+        const float2 ky = pk2(a.ky[q]);
+        const float2 re = psub(x[sl].re, pmul(ky, y[sl].im)), im = pfma(ky, y[sl].re, x[sl].im);
+        dA[(size_t)q * g.K1] = make_float2(re.x, im.x);
+        dB[(size_t)q * g.K1] = make_float2(re.y, im.y);
       }
     }
   }
@@ -408,9 +427,10 @@ __device__ __forceinline__ void xpass_body(const StageArgs& a, int S, int iters,
       if (t < 0 || t >= N3 || (f == 1 && !g.dim3)) {
         for (int k = lane; k < K1; k += 32) d[k] = make_float2(0.f, 0.f);
       } else {
-        const float2* src = g.dim3 ? a.mixin + (((size_t)(rr * 4 + f) * N3 + t) * g.N2 + y) * K1
+        const float2* src = g.dim3 ? a.mixin + mix_pair(g, rr * 2, mix_in_pair(f), mix_in_side(f), t, y)
                                    : a.S + ((size_t)(rr * 5 + f) * N3 + t) * g.Pp;
-        for (int k = lane; k < K1; k += 32) cp_async8(d + k, src + k);
+        const int ks = g.dim3 ? 2 : 1;   // two fields side by side
+        for (int k = lane; k < K1; k += 32) cp_async8(d + k, src + ks * k);
       }
     }
   };
@@ -600,10 +620,12 @@ __device__ __forceinline__ void xpass_body(const StageArgs& a, int S, int iters,
       const float2 c2y = cscale(H(P_S22, s, k), -1.f);
       const float2 c3y = cscale(H(P_P3Y, s, k), -1.f);
       const float2 cBy = cscale(H(P_SB2, s, k), -1.f);
-      float2* m = a.mixout + (((size_t)run * 8 * N3 + t) * g.N2 + y) * K1 + k;
+      float4* m = reinterpret_cast<float4*>(a.mixout) + (((size_t)run * 4 * N3 + t) * g.N2 + y) * K1 + k;
       const size_t cs = g.mblk;
-      m[0 * cs] = c1; m[1 * cs] = c1y; m[2 * cs] = c2; m[3 * cs] = c2y;
-      m[4 * cs] = c3; m[5 * cs] = c3y; m[6 * cs] = cB; m[7 * cs] = cBy;
+      m[0 * cs] = make_float4(c1.x, c1.y, cB.x, cB.y);
+      m[1 * cs] = make_float4(c1y.x, c1y.y, cBy.x, cBy.y);
+      m[2 * cs] = make_float4(c2.x, c2.y, c3.x, c3.y);
+      m[3 * cs] = make_float4(c2y.x, c2y.y, c3y.x, c3y.y);
     }
   }
 
@@ -1340,7 +1362,7 @@ static void ify_launch(const StageArgs& a, int nz, cudaStream_t st) {
 template <int N2>
 static void fy_launch(const StageArgs& a, cudaStream_t st) {
   const int nl = a.nlvl > 0 ? a.nlvl : a.g.N3 - a.lvl0;
-  k_fft_y<N2><<<dim3(cdiv(a.g.K1, ycols<N2>()), nl, a.g.nrun * 4), kYThreads, 0, st>>>(a);
+  k_fft_y<N2><<<dim3(cdiv(a.g.K1, ypcols<N2>()), nl, a.g.nrun * 2), kYThreads, 0, st>>>(a);
 }
 static void launch_ifft_y_z(const StageArgs& a, int nz, cudaStream_t st) {
   switch (a.g.N2) {

@@ -14,7 +14,7 @@ struct XMShape : XMT<N1> {
   // point, a ring: this level and the one below), those of the base (MODE 1,
   // 2), the transpose buffer, the carried combinations ((c1, cB), (c2, c3) per
   // kept slot and lane; 2D: c3 alone in the second) and the staged input rows
-  // of the next level (4 or 3 x K1, and the base run's)
+  // of the next level (2 rows of pairs or 3 rows x K1, and the base run's)
   static constexpr int ROWS = D3 ? 4 : 3;
   static constexpr size_t group_bytes =
       (sizeof(float4) * (size_t)((MODE ? 4 : 2) * N1 + T::TB + 2 * T::NKS * T::G) +
@@ -60,7 +60,7 @@ __device__ __forceinline__ void xmarch_rows(const StageArgs& a, unsigned char* x
   float4* bring = ring + 2 * N1;                    // MODE 1, 2: the base's (U_ in u1)
   float4* tbuf = ring + (MODE ? 4 : 2) * N1;        // transpose buffer
   float4* cbuf = tbuf + T::TB;                      // [2][NKS][G]: (c1, cB), (c2, c3) awaiting their z terms
-  float2* stg = reinterpret_cast<float2*>(cbuf + 2 * NKS * G);   // [ROWS][K1]: u1, u3, b, u2 of the next level; then the base run's
+  float2* stg = reinterpret_cast<float2*>(cbuf + 2 * NKS * G);   // 3D [2][K1] pairs (u1, u3), (b, u2) of the next level, 2D [3][K1] u1, u3, b; then the base run's
   const int partner_lane = (lane & ~(G - 1)) | ((G - l) & (G - 1));
   // the first-stage twiddles of the 128- and 256-point transforms, held in registers
   float4 w1[8];
@@ -104,24 +104,34 @@ __device__ __forceinline__ void xmarch_rows(const StageArgs& a, unsigned char* x
     const float* __restrict__ Ub = a.Ubar + (size_t)run * N3;
     const float* __restrict__ UbB = a.Ubar + (size_t)brun * N3;
     const size_t tstride = D3 ? (size_t)N2 * K1 : (size_t)g.Pp, fstride = (size_t)N3 * tstride;
-    // rows u1, u3, b, u2 at src + field * fstride + t * tstride
-    const float2* __restrict__ src = D3 ? a.mixin + (size_t)run * 4 * fstride + (size_t)y * K1 : a.S + (size_t)run * 5 * fstride;
+    // 3D: rows of pairs at src + 2 (pair * fstride + t * tstride); 2D: rows at src + field * fstride + t * tstride
+    const float2* __restrict__ src = D3 ? a.mixin + 2 * ((size_t)run * 2 * fstride + (size_t)y * K1) : a.S + (size_t)run * 5 * fstride;
     const float2* __restrict__ bsrc =
-        D3 ? a.mixin + (size_t)brun * 4 * fstride + (size_t)y * K1 : a.S + (size_t)brun * 5 * fstride;
-    float2* __restrict__ dst = D3 ? a.mixout + (size_t)run * 8 * fstride + (size_t)y * K1 : a.rnl + (size_t)run * 4 * fstride;
+        D3 ? a.mixin + 2 * ((size_t)brun * 2 * fstride + (size_t)y * K1) : a.S + (size_t)brun * 5 * fstride;
+    float2* __restrict__ dst = D3 ? a.mixout + 2 * ((size_t)run * 4 * fstride + (size_t)y * K1) : a.rnl + (size_t)run * 4 * fstride;
     const float* __restrict__ bnod = MODE == 1 ? a.base + ((size_t)run * 4 * N3 * N2 + y) * N1 : nullptr;
 
-    // the input rows of level t into the stage, 8-byte asynchronous
-    // copies (a row of K1 complex values is not 16-byte aligned in general)
+    // the input rows of level t into the stage by asynchronous copies (16
+    // bytes for a pair, 8 in 2D, where a row of K1 complex values is not
+    // 16-byte aligned in general)
     auto prefetch = [&](int t) {
       if (t < 0 || t >= N3) return;
+      constexpr int R = D3 ? 2 : 3;
 #pragma unroll
-      for (int i = 0; i < (MODE == 2 ? 2 : 1) * ROWS; i++) {
-        const int r = i % ROWS, f = r == 0 ? 0 : (r == 1 ? 2 : (r == 2 ? 3 : 1));
-        const float2* sf = (i < ROWS ? src : bsrc) + f * fstride + (size_t)t * tstride + l;
+      for (int i = 0; i < (MODE == 2 ? 2 : 1) * R; i++) {
+        const int r = i % R;
+        const float2* sf = (i < R ? src : bsrc);
+        if (D3) {
+          sf += 2 * (r * fstride + (size_t)t * tstride + l);
 #pragma unroll
-        for (int j = 0; j < (K1 + G - 1) / G; j++)
-          if (l + G * j < K1) xm_cp8(stg + i * K1 + l + G * j, sf + G * j);
+          for (int j = 0; j < (K1 + G - 1) / G; j++)
+            if (l + G * j < K1) xm_cp16(stg + 2 * (i * K1 + l + G * j), sf + 2 * G * j);
+        } else {
+          sf += (r == 0 ? 0 : r + 1) * fstride + (size_t)t * tstride + l;
+#pragma unroll
+          for (int j = 0; j < (K1 + G - 1) / G; j++)
+            if (l + G * j < K1) xm_cp8(stg + i * K1 + l + G * j, sf + G * j);
+        }
       }
     };
     // this lane's kept mode in kept slot i
@@ -129,10 +139,12 @@ __device__ __forceinline__ void xmarch_rows(const StageArgs& a, unsigned char* x
     // c1, cB and c2, c3 of the last level, awaiting their z terms, per kept slot
     auto Ca = [&](int i) -> float4& { return cbuf[i * G + l]; };
     auto Cb = [&](int i) -> float4& { return cbuf[(NKS + i) * G + l]; };
-    // combination c: 3D 0 c1, 1 c1y, 2 c2, 3 c2y, 4 c3, 5 c3y, 6 cB, 7 cBy; 2D the fields 0 r1, 2 r3, 3 rB
-    auto store = [&](int c, int lvl, int i, float2 v) {
-      const int cc = D3 ? c : (c == 0 ? 0 : (c == 4 ? 2 : 3));
-      if (D3 || (lvl < t_hi && lvl >= t_lo)) dst[(size_t)cc * fstride + (size_t)lvl * tstride + kk(i)] = v;
+    // 3D: the pair p of combinations; 2D: field f (r1, r3, rB) alone
+    auto store2 = [&](int p, int lvl, int i, float2 v, float2 w) {
+      reinterpret_cast<float4*>(dst)[(size_t)p * fstride + (size_t)lvl * tstride + kk(i)] = make_float4(v.x, v.y, w.x, w.y);
+    };
+    auto store = [&](int f, int lvl, int i, float2 v) {
+      if (lvl < t_hi && lvl >= t_lo) dst[(size_t)f * fstride + (size_t)lvl * tstride + kk(i)] = v;
     };
     auto mikx = [&](float k, float2 v) { return make_float2(k * v.y, -k * v.x); };   // -(i k) v
 
@@ -150,7 +162,6 @@ __device__ __forceinline__ void xmarch_rows(const StageArgs& a, unsigned char* x
       // N1 - n at n > N1 - K1, zero between; one load per field from the
       // mode index and a sign, so no position loads two rows
       auto rows = [&](c2x (&x)[E], const float2* st) {
-        const float2 *su1 = st, *su3 = st + K1, *sb = st + 2 * K1, *su2 = st + 3 * K1;
 #pragma unroll
         for (int e = 0; e < E; e++) {
           if (G * e >= K1 && G * e + G - 1 <= N1 - K1) {   // zero at every lane
@@ -163,7 +174,18 @@ __device__ __forceinline__ void xmarch_rows(const StageArgs& a, unsigned char* x
           const float on = (dir || cnj) ? 1.f : 0.f;
           const float sg = dir ? -1.f : 1.f;                 // A.x + sg B.y, B.x - sg A.y
           const float im0 = (n == 0) ? 0.f : on;             // k = 0: real parts only
-          const float2 A = su1[m], B = su3[m], C_ = sb[m], D = D3 ? su2[m] : make_float2(0.f, 0.f);
+          float2 A, B, C_, D = make_float2(0.f, 0.f);
+          if (D3) {
+            const float4 p = reinterpret_cast<const float4*>(st)[m], q = reinterpret_cast<const float4*>(st)[K1 + m];
+            A = make_float2(p.x, p.y);
+            B = make_float2(p.z, p.w);
+            C_ = make_float2(q.x, q.y);
+            D = make_float2(q.z, q.w);
+          } else {
+            A = st[m];
+            B = st[K1 + m];
+            C_ = st[2 * K1 + m];
+          }
           const float2 re = make_float2(on * A.x + (sg * im0) * B.y, on * C_.x + (sg * im0) * D.y);
           const float2 im = make_float2(on * B.x - (sg * im0) * A.y, on * D.x - (sg * im0) * C_.y);
           x[e] = c2x{re, im};
@@ -245,8 +267,8 @@ __device__ __forceinline__ void xmarch_rows(const StageArgs& a, unsigned char* x
 
       // the forward transform pairs of the step, one batch at a time:
       //   3D b = 0: Q1 + i QB, Q2 + i P4 (level t-1)   [1 <= k <= n + 1]
-      //      b = 1: S1 + i SB1, S12 + i S22            [k <= n]
-      //      b = 2: P3 + i P3Y, SB2                    [k <= n]
+      //      b = 1: S1 + i SB1, S12 + i SB2            [k <= n]
+      //      b = 2: P3 + i P3Y, S22                    [k <= n]
       //   2D b = 0: Q1 + i QB, P4 (level t-1)
       //      b = 1: S1 + i SB1, P3
       const int nb = k <= n ? (D3 ? 3 : 2) : 1;
@@ -285,23 +307,23 @@ __device__ __forceinline__ void xmarch_rows(const StageArgs& a, unsigned char* x
           for (int s = 0; s < E; s++) {
             const float4 cv = curl[s * G + l + tok];
             const float U1 = cv.x, Bv = cv.y, U2 = cv.w;
-            float s1, sb1, s12, s22;
+            float s1, sb1, s12, sb2;
             float4 bc;
             if (MODE == 0) {
               const float u1t = U1 + ub;
               s1 = U1 * (U1 + 2.f * ub);
               sb1 = u1t * Bv;
               s12 = u1t * U2;
-              s22 = U2 * U2;
+              sb2 = U2 * Bv;
             } else {
               bc = bcur[s * G + l + tok];
               s1 = (2.f * U1) * bc.x;
               sb1 = Bv * bc.x + bc.y * U1;
               s12 = U1 * bc.w + bc.x * U2;
-              s22 = (2.f * U2) * bc.w;
+              sb2 = Bv * bc.w + bc.y * U2;
             }
             if (D3) {
-              z[T::pos(s)] = c2x{make_float2(s1, s12), make_float2(sb1, s22)};
+              z[T::pos(s)] = c2x{make_float2(s1, s12), make_float2(sb1, sb2)};
             } else {
               const float4 pv = prev[s * G + l + tok];
               const float w3 = lof * cv.z;
@@ -319,21 +341,21 @@ __device__ __forceinline__ void xmarch_rows(const StageArgs& a, unsigned char* x
 #pragma unroll
           for (int s = 0; s < E; s++) {
             const float4 pv = prev[s * G + l + tok], cv = curl[s * G + l + tok];
-            const float U1 = cv.x, Bv = cv.y, U3 = cv.z, U2 = cv.w;
+            const float U1 = cv.x, U3 = cv.z, U2 = cv.w;
             const float w3 = lof * U3;
-            float p3 = tdi * U1 + tlo * pv.x, p3y = tdi * U2 + tlo * pv.w, sb2;
+            float p3 = tdi * U1 + tlo * pv.x, p3y = tdi * U2 + tlo * pv.w, s22;
             if (MODE == 0) {
               p3 = (p3 + (tlo * ubm + tdi * ub)) * w3;
               p3y *= w3;
-              sb2 = U2 * Bv;
+              s22 = U2 * U2;
             } else {
               const float4 bp = bprev[s * G + l + tok], bc = bcur[s * G + l + tok];
               const float W3 = lof * bc.z;
               p3 = pr(p3, w3, tdi * bc.x + tlo * bp.x, W3);
               p3y = pr(p3y, w3, tdi * bc.w + tlo * bp.w, W3);
-              sb2 = Bv * bc.w + bc.y * U2;
+              s22 = (2.f * U2) * bc.w;
             }
-            z[T::pos(s)] = c2x{make_float2(p3, sb2), make_float2(p3y, 0.f)};
+            z[T::pos(s)] = c2x{make_float2(p3, s22), make_float2(p3y, 0.f)};
           }
         }
         T::template fft<false>(z, tbuf, tw4, tw2, l, w1);
@@ -360,31 +382,36 @@ __device__ __forceinline__ void xmarch_rows(const StageArgs& a, unsigned char* x
             const float2 P4 = D3 ? B2 : B1;
             if (fin) {
               const float4 ca = Ca(i), cb = Cb(i);
-              store(0, tm, i, make_float2(ca.x - fu * A1.x, ca.y - fu * A1.y));
-              store(6, tm, i, make_float2(ca.z - fu * A2.x, ca.w - fu * A2.y));
-              if (D3) store(2, tm, i, make_float2(cb.x - fu * B1.x, cb.y - fu * B1.y));
-              store(4, tm, i, make_float2(cb.z - fd * P4.x, cb.w - fd * P4.y));
+              const float2 c1 = make_float2(ca.x - fu * A1.x, ca.y - fu * A1.y);
+              const float2 cB = make_float2(ca.z - fu * A2.x, ca.w - fu * A2.y);
+              const float2 c3 = make_float2(cb.z - fd * P4.x, cb.w - fd * P4.y);
+              if (D3) {
+                store2(0, tm, i, c1, cB);
+                store2(2, tm, i, make_float2(cb.x - fu * B1.x, cb.y - fu * B1.y), c3);
+              } else {
+                store(0, tm, i, c1);
+                store(2, tm, i, c3);
+                store(3, tm, i, cB);
+              }
             }
             Ca(i) = make_float4(-sd * A1.x, -sd * A1.y, -sd * A2.x, -sd * A2.y);
             Cb(i) = make_float4(-sd * B1.x, -sd * B1.y, -sl * P4.x, -sl * P4.y);
-          } else if (b == 1) {   // 3D S1, SB1, S12, S22; 2D S1, SB1, P3
+          } else if (b == 1) {   // 3D S1, SB1, S12, SB2; 2D S1, SB1, P3
             const float k = __ldg(a.kx + kk(i));
             const float2 a1 = mikx(k, A1), aB = mikx(k, A2), a2 = mikx(k, B1);
             const float4 ca = Ca(i), cb = Cb(i);
             Ca(i) = make_float4(a1.x + ca.x, a1.y + ca.y, aB.x + ca.z, aB.y + ca.w);
             if (D3) {
               Cb(i) = make_float4(a2.x + cb.x, a2.y + cb.y, cb.z, cb.w);
-              store(1, t, i, make_float2(-B1.x, -B1.y));
-              store(3, t, i, make_float2(-B2.x, -B2.y));
+              store2(1, t, i, make_float2(-B1.x, -B1.y), make_float2(-B2.x, -B2.y));
             } else {
               Cb(i) = make_float4(0.f, 0.f, cb.z + a2.x, cb.w + a2.y);
             }
-          } else {   // P3, P3Y, SB2
+          } else {   // P3, P3Y, S22
             const float2 a3 = mikx(__ldg(a.kx + kk(i)), A1);
             const float4 cb = Cb(i);
             Cb(i) = make_float4(cb.x, cb.y, cb.z + a3.x, cb.w + a3.y);
-            store(5, t, i, make_float2(-A2.x, -A2.y));
-            store(7, t, i, make_float2(-B1.x, -B1.y));
+            store2(3, t, i, make_float2(-B1.x, -B1.y), make_float2(-A2.x, -A2.y));
           }
         }
         tok = __float_as_int(z[0].re.x) & rz;

@@ -102,6 +102,10 @@ __device__ __forceinline__ void xm_cp8(void* smem, const void* gmem) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem));
 }
+__device__ __forceinline__ void xm_cp16(void* smem, const void* gmem) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem));
+}
 __device__ __forceinline__ void xm_cp_wait() { asm volatile("cp.async.wait_all;\n" ::); }
 
 __device__ __forceinline__ float4 c2x_f4(const c2x& v) { return make_float4(v.re.x, v.re.y, v.im.x, v.im.y); }
