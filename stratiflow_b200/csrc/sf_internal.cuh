@@ -5,7 +5,8 @@
 //                                       stage k reads one and writes the other
 //   rold            [nrun][4][N3][Pp]   explicit terms r1,r2,r3,rB of the last
 //                                       stage (the zeta term of ExplicitRK)
-//   rnl             [nrun][4][N3][Pp]   nonlinear terms of this stage
+//   rnl             [nrun][4][N3][Pp]   nonlinear terms of this stage (with
+//                                       k_z_step_f the two take turns)
 //   qbuf            [nrun][N3][Pp]      forward-sweep scratch of the pressure solve
 //   mixin  (3D)     [nrun][2][N3][N2][K1][2]  fields after the inverse y
 //                   transform, two side by side: (u1, u3), (b, u2)

@@ -219,7 +219,16 @@ static int refactor(sf_solver* s) {
   return SF_OK;
 }
 
+// fused: the z pass is k_z_step_f's, between whose stages the two buffers of
+// explicit terms take turns (the other z kernels copy them)
+static StageArgs stage_args(sf_solver* s, int k, int cur, bool linear, bool fused);
 static StageArgs stage_args(sf_solver* s, int k, int cur, bool linear) {
+  StageArgs z{};
+  z.zkernel = s->zkernel;
+  z.g = s->g;
+  return stage_args(s, k, cur, linear, z_step_takes_c(z) && zstep_f_supported(s->g));
+}
+static StageArgs stage_args(sf_solver* s, int k, int cur, bool linear, bool fused) {
   StageArgs a{};
   a.g = s->g;
   a.S = s->S[cur];
@@ -262,6 +271,7 @@ static StageArgs stage_args(sf_solver* s, int k, int cur, bool linear) {
   a.cv = 0.5f * h / (float)s->Re;
   a.cb = 0.5f * h / (float)s->Re / (float)s->Pr;
   a.pm = 1.0f / h;             // RemoveDivergence(1/h[k])
+  if (fused && k == 1) std::swap(a.rnl, a.rold);
   return a;
 }
 
@@ -1126,7 +1136,7 @@ int sf_ensemble_step(sf_ensemble* e, int nsteps) {
       for (int r = 0; r < R; r++) {
         StageArgs a;
         std::memset(&a, 0, sizeof(a));   // the padding too: the copies are compared as bytes
-        a = stage_args(e->members[r], k, cur, false);
+        a = stage_args(e->members[r], k, cur, false, e->members[r]->g.N3 <= kEnsFusedN3);
         StageArgs& h = e->h_args[((size_t)p * 3 + k) * R + r];
         changed = changed || std::memcmp(&h, &a, sizeof(a)) != 0;
         std::memcpy(&h, &a, sizeof(a));

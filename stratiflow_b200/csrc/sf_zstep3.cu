@@ -30,23 +30,26 @@ constexpr ZfKernel zf_kernel() {
 
 // Measured per launch (us), k_z_step_c in brackets; "many" has more blocks
 // of 8 modes than the GPU has SMs:
-//   3D  short    64x32x64        12.2 (29.7)
-//       one      64x32x96        16.3 (34.8), two 18.2;    32x16x332 27.8 (63.7), two 44.4
-//                256x128x384    169.6 (179.8), two 211 (two blocks do not fit one SM)
-//       two      2 x 128x64x180  47.2 (84.5), one 55.4;    256x128x128 67.6 (72.7), one 89.4
-//   2D  short4   64x1x64         11.6 (26.1), short8 13.8
-//       short8   128x1x128       14.4 (32.7), one 16.7;    32 x 128x1x128 23.9 (32.7), many 26.3
+//   3D  short4   64x32x64        10.5 (29.7)
+//       short8   64x32x96        12.8 (34.8), one 16.3;    128x64x96 19.1, two 22.0
+//       mid      64x32x128       15.1, one 20.8;           3 x 64x64x128 32.2, two 37.1; 256x128x128 72, two 67
+//       one      32x16x332       27.8 (63.7), two 44.4;    256x128x384 174 (180), two 211 (two blocks do not fit one SM)
+//       two      2 x 128x64x180  46 (84.5), one 55.4;      256x128x128 67 (72.7), one 89.4
+//   2D  short4   64x1x64         10.2 (26.1)
+//       short8   128x1x128       12.4 (32.7), one 16.7;    32 x 128x1x128 19.8 (32.7), many 26.3
 //       one      6 x 512x1x388   26.9 (61.5), many 43.5;   64 x 256x1x384 130 (143), many 188
 //       many     64 x 256x1x256  89.3 (101), one 99.8;     8 x 512x1x256 32.5 (40.5), one 36.3
 //       tall     as "one" where its columns do not fit: 64 x 256x1x384 125
 // Two blocks of an SM only pay where the SM's L1 keeps some of its room and
 // the second block has something to do; with one block each lane may hold
 // more levels' loads in flight.
-constexpr ZfKernel k3short = zf_kernel<4, 4, 4, 1, 4, false, false, false, 1>();
+constexpr ZfKernel k3short4 = zf_kernel<4, 4, 4, 1, 4, false, false, false, 1>();
+constexpr ZfKernel k3short8 = zf_kernel<4, 3, 8, 2, 8, false, false, false, 1>();
+constexpr ZfKernel k3mid = zf_kernel<4, 4, 8, 2, 8, false, false, false, 1>();
 constexpr ZfKernel k3one = zf_kernel<4, 4, 0, 12, 4, true, false, false, 1>();
 constexpr ZfKernel k3two = zf_kernel<4, 3, 0, 8, 3, true, false, false, 2>();
-constexpr ZfKernel k2short4 = zf_kernel<3, 4, 4, 2, 4, false, false, false, 2>();
-constexpr ZfKernel k2short8 = zf_kernel<3, 8, 4, 2, 4, false, false, false, 1>();
+constexpr ZfKernel k2short4 = zf_kernel<3, 4, 4, 2, 4, false, false, false, 1>();
+constexpr ZfKernel k2short8 = zf_kernel<3, 4, 8, 3, 8, false, false, false, 1>();
 constexpr ZfKernel k2one = zf_kernel<3, 4, 0, 12, 4, true, true, true, 1>();
 constexpr ZfKernel k2many = zf_kernel<3, 4, 0, 8, 2, true, false, false, 2>();
 constexpr ZfKernel k2tall = zf_kernel<3, 8, 0, 9, 2, true, false, false, 1>();
@@ -63,10 +66,13 @@ bool zf_takes(const ZfKernel& k, int N3, size_t room = kSmem1) {
 // the shape for a grid; null: too tall for every shape (k_z_step_c runs). The
 // z-chunk setting's 8 and 16 ask for more and for fewer blocks per SM
 const ZfKernel* zf_pick(const Geo& g, int zchunks) {
-  const bool many = zchunks ? zchunks == 8 : (long long)((g.P + kFM - 1) / kFM) * g.nrun > 148;
+  const long long blocks = (long long)((g.P + kFM - 1) / kFM) * g.nrun;
+  const bool many = zchunks ? zchunks == 8 : blocks > 148;
   const int N3 = g.N3;
   if (g.dim3) {
-    if (zf_takes(k3short, N3)) return &k3short;
+    if (zf_takes(k3short4, N3)) return &k3short4;
+    if (zf_takes(k3short8, N3)) return &k3short8;
+    if (blocks <= 4 * 148 && zf_takes(k3mid, N3)) return &k3mid;
     if (many && zf_takes(k3two, N3, kSmem2)) return &k3two;
     return zf_takes(k3one, N3) ? &k3one : nullptr;
   }
@@ -88,7 +94,7 @@ int launch_z_step_f(const StageArgs& a, cudaStream_t st) {
 }
 
 int prepare_zstep_f_kernels() {
-  for (const ZfKernel* k : {&k3short, &k3one, &k3two, &k2short4, &k2short8, &k2one, &k2many, &k2tall})
+  for (const ZfKernel* k : {&k3short4, &k3short8, &k3mid, &k3one, &k3two, &k2short4, &k2short8, &k2one, &k2many, &k2tall})
     if (cudaFuncSetAttribute(k->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem1) != cudaSuccess) return -1;
   return 0;
 }

@@ -16,13 +16,18 @@
 //
 // 8 modes are 64 bytes of a level's row (two whole sectors); twice as many
 // blocks as with 16 modes leave fewer SMs idle and a last wave half as long.
-// Chunks of up to L = 4 levels live in registers (every input loaded at once,
+// Chunks of up to L = 4 or 8 levels live in registers (every input loaded at once,
 // be_j and the pivots never reloaded); longer ones keep be_j / D_j in the
 // block's shared rows and load the pivots again in each sweep, L = 0. What
 // remains is the latency of those loads, about 1900 cycles under load at
 // 256x128x384: fewer, larger batches are worth more than more warps (two
 // blocks of 16 warps there take 243-290 us, one with twice the levels in
 // flight 170).
+//
+// r_old: the buffers of r take turns over a step's stages, so nothing is copied
+// for the next stage's zeta term (its own buffer was written each stage: 4 of
+// 24 field-sized transfers); u3's and b's r are completed in place by the
+// linear buoyancy terms, in the stages that another follows.
 //
 // The arithmetic of every term is k_z_step_c's, in the same order; the chunks
 // are others, so the two agree to rounding.
@@ -153,9 +158,12 @@ __device__ __forceinline__ ZfMap zf_rhs(const StageArgs& a, const ZfLane& t, con
   const float2* __restrict__ uc = Sr + F * FB;
   const float2* __restrict__ xc = Sr + (FAM == 2 ? 2 : 3) * FB;   // b for u3, u3 for b
   const float2* __restrict__ pc = Sr + 4 * FB;
-  const float2* __restrict__ rc = a.rnl + (size_t)(t.run * 4 + F) * FB;
-  float2* rold = a.rold + (size_t)(t.run * 4 + F) * FB;
+  float2* rc = a.rnl + (size_t)(t.run * 4 + F) * FB;
+  const float2* __restrict__ rold = a.rold + (size_t)(t.run * 4 + F) * FB;
   const bool use_rold = (a.hz != 0.f);
+  // the next stage reads this stage's explicit terms from where they lie (the
+  // solver's two buffers take turns); only those of u3 and b are not yet whole
+  const bool keep = F >= 2 && a.stage < 2 && !a.adjoint;
   const float kgrad = (F == 0) ? t.kxv : t.kyv;
   const float2 *Uc = F == 2 ? Wc : Bc, *Xc = F == 2 ? Bc : Wc;   // COL: this field's column, and the other's
   constexpr bool UC = COL && F >= 2;
@@ -230,7 +238,7 @@ __device__ __forceinline__ ZfMap zf_rhs(const StageArgs& a, const ZfLane& t, con
       } else if (in) {
         X[j * kFM] = be;
       }
-      if (in && t.act) rold[j * Pp + m] = rt;
+      if (keep && in && t.act) rc[j * Pp + m] = rt;
       const float2 B = cfma(al, map.B, be);
       map.A = in ? map.A * al : map.A;
       map.B = in ? B : map.B;

@@ -21,8 +21,9 @@ GRIDS = [
     (64, 1, 132, 50), (64, 1, 268, 50), (64, 1, 272, 50),                     # 2D, blocks for two per SM, and past it
     (64, 1, 492, 1), (32, 1, 824, 1), (32, 1, 828, 1),                        # 2D, tall, and past every shape
     (16, 16, 32, 1), (16, 16, 64, 2),                                         # 3D in registers
-    (16, 16, 68, 1), (16, 16, 332, 1), (16, 16, 672, 1), (16, 16, 676, 1),    # 3D, one block per SM, and past it
-    (16, 16, 68, 26), (32, 16, 332, 15), (32, 16, 336, 15),                   # 3D, blocks for two per SM, and past it
+    (16, 16, 96, 1), (16, 16, 100, 2), (16, 16, 128, 1), (16, 16, 100, 99),   # 3D, the longer register chunks, and past the block rule
+    (16, 16, 68, 1), (16, 16, 132, 1), (16, 16, 332, 1), (16, 16, 672, 1), (16, 16, 676, 1),    # 3D, one block per SM, and past it
+    (16, 16, 132, 26), (32, 16, 332, 15), (32, 16, 336, 15),                   # 3D, blocks for two per SM, and past it
 ]
 
 
