@@ -31,7 +31,7 @@ static_assert(kEnsThreads == ZfShape<3, 4>::THREADS, "a z item is three fields o
 
 // warps that march in a block of one grid width (as many as the shared memory takes)
 template <int N1>
-constexpr int ens_warps() { return std::min(kEnsWarps, XMShape<N1, false, 0>::WARPS); }
+constexpr int ens_warps() { return std::min(kEnsWarps, XMShape<N1, false, 0, false>::WARPS); }
 
 template <int N1>
 __device__ __forceinline__ void ens_x(const StageArgs& a, unsigned char* sm, const EnsItem& it, bool tables) {
@@ -41,7 +41,7 @@ __device__ __forceinline__ void ens_x(const StageArgs& a, unsigned char* sm, con
   }
   const int w = threadIdx.x >> 5;
   const StageArgs la = a;   // out of shared memory, which the march's stores might alias
-  if (w < it.iters) xmarch_rows<N1, false, 0>(la, sm, 1, 0, a.g.N3, it.S, it.x + w, it.x + w + 1);
+  if (w < it.iters) xmarch_rows<N1, false, 0, false>(la, sm, 1, 0, a.g.N3, it.S, it.x + w, it.x + w + 1);
 }
 
 __global__ void __launch_bounds__(kEnsThreads, 1) k_ens_stage(const StageArgs* __restrict__ args,
@@ -145,12 +145,12 @@ int ensemble_x_rows(int N1) {
 size_t ensemble_smem(int N1, int N3) {
   size_t x = 0;
   switch (N1) {
-    case 16: x = XMShape<16, false, 0>::smem(ens_warps<16>()); break;
-    case 32: x = XMShape<32, false, 0>::smem(ens_warps<32>()); break;
-    case 64: x = XMShape<64, false, 0>::smem(ens_warps<64>()); break;
-    case 128: x = XMShape<128, false, 0>::smem(ens_warps<128>()); break;
-    case 256: x = XMShape<256, false, 0>::smem(ens_warps<256>()); break;
-    default: x = XMShape<512, false, 0>::smem(ens_warps<512>()); break;
+    case 16: x = XMShape<16, false, 0, false>::smem(ens_warps<16>()); break;
+    case 32: x = XMShape<32, false, 0, false>::smem(ens_warps<32>()); break;
+    case 64: x = XMShape<64, false, 0, false>::smem(ens_warps<64>()); break;
+    case 128: x = XMShape<128, false, 0, false>::smem(ens_warps<128>()); break;
+    case 256: x = XMShape<256, false, 0, false>::smem(ens_warps<256>()); break;
+    default: x = XMShape<512, false, 0, false>::smem(ens_warps<512>()); break;
   }
   const size_t z = N3 > kEnsFusedN3 ? zc_smem_bytes<2 * kEnsWarps>(N3)
                                     : ZfShape<3, 4>::smem(N3, N3 > 64, N3 > 64);

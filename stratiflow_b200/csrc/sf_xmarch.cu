@@ -1,26 +1,32 @@
-// The 3D x pass of the nonlinear step as level-marching lane groups
-// (BuildRHS, IMEXRK.cpp:136-193: ToNodal's x part, the nodal products, ToModal's
-// x part with 1/(N1 N2) and the 2/3 truncation, then the x derivatives and the
-// z stencils that follow each product).
+// The x pass as level-marching lane groups (BuildRHS, IMEXRK.cpp:136-193:
+// ToNodal's x part, the nodal products, ToModal's x part with 1/(N1 N2) and the
+// 2/3 truncation, then the x derivatives and the z stencils that follow each
+// product; and the same about a base flow).
 //
-// One lane group (XMT<N1>::G lanes: the whole warp at N1 = 256, else
-// FFTShape<N1>::G lanes) owns one y row and walks up a range of z levels. At level t it inverse-transforms the four fields of level t
-// (u1 + i u3 and b + i u2, packed as one two-transform pair, sf_fft2.cuh),
-// keeps them in registers and the fields of level t-1 in its own shared
-// memory, forms the eleven products of level t (with P4 of level t-1, the one
-// product that needs u3 of the level above), forward-transforms them as three
-// packed pairs and finishes the combinations:
+// One lane group (XMT<N1>::G lanes) owns one row, a y row in 3D, and walks up a
+// range of z levels. At level t it inverse-transforms the fields of level t
+// (u1 + i u3 and b + i u2, packed as one two-transform pair, sf_xmt.cuh), keeps
+// them in registers and the fields of level t-1 in its own shared memory, forms
+// the eleven products of level t (with P4 of level t-1, the one product that
+// needs u3 of the level above), forward-transforms them as three packed pairs
+// and finishes the combinations:
 //   level t-1: c1, cB, c2 get their ddz(D->N) term from Q1, QB, Q2 of level t,
 //              c3 its ddz(N->D) term from P4 of level t-1; written out;
 //   level t:   c1y, c2y, c3y, cBy written out; c1, cB, c2, c3 started and
-//              carried in registers to the next level.
+//              carried to the next level.
 // The nodal values a lane forms after the inverse transform are those of the
-// x positions it feeds into the forward transforms (x = l + G e), so the
-// products need no exchange between lanes; the only shared memory traffic is
-// the transforms' transposes, the level below and the staged input rows.
-// No block-wide barrier after set-up: the groups of a warp share their level
-// range (they own neighbouring y rows) and march in step; warps are
-// independent.
+// x positions it feeds into the forward transforms, so the products need no
+// exchange between lanes; the only shared memory traffic is the transforms'
+// transposes, the level below and the staged input rows. No block-wide barrier
+// after set-up: the groups of a warp march in step, warps are independent.
+//
+// The shared-memory pipe bounds it (82 to 89 % busy at 256x128x384). So the
+// nonlinear step carries its combinations in registers where a lane keeps three
+// modes or fewer, and forms the first batch of products from the inverse
+// transform's own registers: 230 us a stage with both in shared memory, 208
+// with the first, 197 with both; 2 x 128x64x180: 66, 61, 58; 32 x 256x256 in 2D:
+// 43, 41, 36. The linear and tangent modes need the base flow's registers too:
+// carried there as well, they gained 3 % at some sizes and lost 4 % at others.
 #include "sf_xmarch.cuh"
 
 namespace sf {

@@ -7,7 +7,10 @@ namespace sf {
 
 // D3: 3D rows (else 2D); MODE 0: BuildRHS; 1: BuildRHSLinear about the frozen
 // nodal base; 2: about the live state of the base run
-template <int N1, bool D3, int MODE>
+// CR: the carried combinations in registers instead of shared memory (where
+// a warp has 168 registers and needs no more; the ensembles' kernel, which
+// holds its z items too, spills: a stage of 64 members 159 us without, 164 with)
+template <int N1, bool D3, int MODE, bool CR = (XMT<N1>::NKS <= 3 && MODE == 0)>
 struct XMShape : XMT<N1> {
   using T = XMT<N1>;
   // shared memory of one row: two levels of nodal values (float4 per x
@@ -17,7 +20,7 @@ struct XMShape : XMT<N1> {
   // of the next level (2 rows of pairs or 3 rows x K1, and the base run's)
   static constexpr int ROWS = D3 ? 4 : 3;
   static constexpr size_t group_bytes =
-      (sizeof(float4) * (size_t)((MODE ? 4 : 2) * N1 + T::TB + 2 * T::NKS * T::G) +
+      (sizeof(float4) * (size_t)((MODE ? 4 : 2) * N1 + T::TB + (CR ? 0 : 2 * T::NKS * T::G)) +
        sizeof(float2) * (MODE == 2 ? 2 : 1) * ROWS * T::K1 + 15) / 16 * 16;
   static constexpr size_t table_bytes = (sizeof(float4) + sizeof(float2)) * (size_t)T::TWE;
   // warps of a block, one block per SM: as many as the shared memory takes,
@@ -42,10 +45,10 @@ __device__ __forceinline__ void xmarch_tables(unsigned char* xsm, const float2* 
 // level). 2D: a unit is W segments of seg levels, one per lane group (the
 // groups of a warp march in step, each on its own segment). The block has
 // filled the tables (and waited); each warp has its own part of xsm.
-template <int N1, bool D3, int MODE>
+template <int N1, bool D3, int MODE, bool CR = (XMT<N1>::NKS <= 3 && MODE == 0)>
 __device__ __forceinline__ void xmarch_rows(const StageArgs& a, unsigned char* xsm, int nruns, int t_lo, int t_hi, int seg,
                                             long long u, const long long uend) {
-  using X = XMShape<N1, D3, MODE>;
+  using X = XMShape<N1, D3, MODE, CR>;
   using T = XMT<N1>;
   constexpr int G = T::G, E = T::E, K1 = T::K1, W = T::W, NKS = T::NKS, ROWS = X::ROWS;
   const Geo& g = a.g;
@@ -60,7 +63,7 @@ __device__ __forceinline__ void xmarch_rows(const StageArgs& a, unsigned char* x
   float4* bring = ring + 2 * N1;                    // MODE 1, 2: the base's (U_ in u1)
   float4* tbuf = ring + (MODE ? 4 : 2) * N1;        // transpose buffer
   float4* cbuf = tbuf + T::TB;                      // [2][NKS][G]: (c1, cB), (c2, c3) awaiting their z terms
-  float2* stg = reinterpret_cast<float2*>(cbuf + 2 * NKS * G);   // 3D [2][K1] pairs (u1, u3), (b, u2) of the next level, 2D [3][K1] u1, u3, b; then the base run's
+  float2* stg = reinterpret_cast<float2*>(cbuf + (CR ? 0 : 2 * NKS * G));   // 3D [2][K1] pairs (u1, u3), (b, u2) of the next level, 2D [3][K1] u1, u3, b; then the base run's
   const int partner_lane = (lane & ~(G - 1)) | ((G - l) & (G - 1));
   // the first-stage twiddles of the 128- and 256-point transforms, held in registers
   float4 w1[8];
@@ -137,8 +140,9 @@ __device__ __forceinline__ void xmarch_rows(const StageArgs& a, unsigned char* x
     // this lane's kept mode in kept slot i
     auto kk = [&](int i) { return T::kmode(l, i); };
     // c1, cB and c2, c3 of the last level, awaiting their z terms, per kept slot
-    auto Ca = [&](int i) -> float4& { return cbuf[i * G + l]; };
-    auto Cb = [&](int i) -> float4& { return cbuf[(NKS + i) * G + l]; };
+    float4 ca_[CR ? NKS : 1], cb_[CR ? NKS : 1];
+    auto Ca = [&](int i) -> float4& { return CR ? ca_[CR ? i : 0] : cbuf[i * G + l]; };
+    auto Cb = [&](int i) -> float4& { return CR ? cb_[CR ? i : 0] : cbuf[(NKS + i) * G + l]; };
     // 3D: the pair p of combinations; 2D: field f (r1, r3, rB) alone
     auto store2 = [&](int p, int lvl, int i, float2 v, float2 w) {
       reinterpret_cast<float4*>(dst)[(size_t)p * fstride + (size_t)lvl * tstride + kk(i)] = make_float4(v.x, v.y, w.x, w.y);
@@ -208,8 +212,8 @@ __device__ __forceinline__ void xmarch_rows(const StageArgs& a, unsigned char* x
           }
       }
       // level t into its ring slot (u1, b, u3, u2 per x point; zero outside 0..N3-1)
+      c2x x[E];   // MODE 0: and kept for the first batch
       if (flow) {
-        c2x x[E];
         xm_cp_wait();
         __syncwarp();
         rows(x, stg);
@@ -239,7 +243,10 @@ __device__ __forceinline__ void xmarch_rows(const StageArgs& a, unsigned char* x
         __syncwarp();
         if (k <= n) prefetch(t + 1);
 #pragma unroll
-        for (int s = 0; s < E; s++) curl[s * G + l] = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int s = 0; s < E; s++) {
+          x[s] = c2x{make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+          curl[s * G + l] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
         if (MODE == 2) {
 #pragma unroll
           for (int s = 0; s < E; s++) bcur[s * G + l] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -272,16 +279,16 @@ __device__ __forceinline__ void xmarch_rows(const StageArgs& a, unsigned char* x
       //   2D b = 0: Q1 + i QB, P4 (level t-1)
       //      b = 1: S1 + i SB1, P3
       const int nb = k <= n ? (D3 ? 3 : 2) : 1;
-#pragma unroll 1
-      for (int b = 0; b < nb; b++) {
+      auto batch = [&](int b, auto first) __attribute__((always_inline)) {
+        constexpr bool F0 = decltype(first)::value;   // b = 0
         c2x z[E];
         // the value of a product of two linear forms: x y, or its derivative
         // about the base, x Y + X y
         auto pr = [&](float x, float y, float X, float Y) { return MODE ? x * Y + X * y : x * y; };
-        if (b == 0) {
+        if (F0) {
 #pragma unroll
           for (int s = 0; s < E; s++) {
-            const float4 pv = prev[s * G + l + tok], cv = curl[s * G + l + tok];   // u1, b, u3, u2 of t-1, t
+            const float4 pv = prev[s * G + l + tok], cv = MODE == 0 ? c2x_f4(x[s]) : curl[s * G + l + tok];   // u1, b, u3, u2 of t-1, t
             const float U1 = cv.x, Bv = cv.y, U3 = cv.z, U2 = cv.w;
             const float w3 = lof * U3;
             float q1 = hb * U1 + hb * pv.x, qb = hb * Bv + hb * pv.y, q2 = hb * U2 + hb * pv.w, p4;
@@ -378,7 +385,7 @@ __device__ __forceinline__ void xmarch_rows(const StageArgs& a, unsigned char* x
           const float2 SI = pmul(padd(zs.im, p.im), SC), DR = pmul(psub(p.re, zs.re), SC);
           const float2 A1 = make_float2(SR.x, DI.x), A2 = make_float2(SI.x, DR.x);   // transform A's products
           const float2 B1 = make_float2(SR.y, DI.y), B2 = make_float2(SI.y, DR.y);   // transform B's
-          if (b == 0) {   // A1 = Q1, A2 = QB; 3D B1 = Q2, B2 = P4 of level t-1; 2D B1 = P4
+          if (F0) {   // A1 = Q1, A2 = QB; 3D B1 = Q2, B2 = P4 of level t-1; 2D B1 = P4
             const float2 P4 = D3 ? B2 : B1;
             if (fin) {
               const float4 ca = Ca(i), cb = Cb(i);
@@ -415,7 +422,10 @@ __device__ __forceinline__ void xmarch_rows(const StageArgs& a, unsigned char* x
           }
         }
         tok = __float_as_int(z[0].re.x) & rz;
-      }
+      };
+      batch(0, std::true_type{});
+#pragma unroll 1
+      for (int b = 1; b < nb; b++) batch(b, std::false_type{});
     }
   }
 }

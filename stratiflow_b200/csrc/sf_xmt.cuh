@@ -19,7 +19,7 @@ struct XMT {   // N1 = 32, 64: two-stage transforms over FFTShape<N1>::G lanes
   static constexpr int TWE = E * G;                 // twiddle table entries
   // output slot of the i-th kept candidate; slot h*G + k2 holds mode l + h*G + E*k2
   __host__ __device__ static constexpr int kslot(int i) { return (i / NK2) * G + i % NK2; }
-  __device__ static int kmode(int l, int i) { return l + (kslot(i) / G) * G + E * (kslot(i) % G); }
+  __device__ __forceinline__ static int kmode(int l, int i) { return l + (kslot(i) / G) * G + E * (kslot(i) % G); }
   // x position index e (x = l + G e) of inverse output slot s
   __host__ __device__ static constexpr int pos(int s) { return s / G + H * (s % G); }
   // slot holding mode N1 - k at lane G - l (l >= 1) or at lane 0 (l = 0)
@@ -28,11 +28,11 @@ struct XMT {   // N1 = 32, 64: two-stage transforms over FFTShape<N1>::G lanes
     const int q = lane0 ? (E - h - H * k2) % E : E - 1 - h - H * k2;
     return (q % H) * G + q / H;
   }
-  __device__ static void fill(float4* tw4, float2* tw2, const float2* tw, int tid, int nthr) {
+  __device__ __forceinline__ static void fill(float4* tw4, float2* tw2, const float2* tw, int tid, int nthr) {
     fill_tw2<N1>(tw4, tw2, tw, tid, nthr);
   }
   template <bool INV>
-  __device__ static void fft(c2x (&x)[E], float4* buf, const float4* tw4, const float2* tw2, int l,
+  __device__ __forceinline__ static void fft(c2x (&x)[E], float4* buf, const float4* tw4, const float2* tw2, int l,
                              const float4 (&)[8]) {
     reg_fft2<N1, INV>(x, buf, tw4, tw2, l);
   }
@@ -45,14 +45,14 @@ struct XMT<128> {   // 16 lanes per row: three stages, 8 x 4 x 4 (reg_fft2_128h)
   // slot of out[l + 16 j]: j = i + 2 q in slot i*4 + q
   __host__ __device__ static constexpr int jslot(int j) { return (j % 2) * 4 + j / 2; }
   __host__ __device__ static constexpr int kslot(int i) { return jslot(i); }
-  __device__ static int kmode(int l, int i) { return l + 16 * i; }
+  __device__ __forceinline__ static int kmode(int l, int i) { return l + 16 * i; }
   __host__ __device__ static constexpr int pos(int s) { return s / 4 + 2 * (s % 4); }
   __host__ __device__ static constexpr int partner(int i, bool lane0) { return jslot(lane0 ? (8 - i) % 8 : 7 - i); }
-  __device__ static void fill(float4* tw4, float2* tw2, const float2* tw, int tid, int nthr) {
+  __device__ __forceinline__ static void fill(float4* tw4, float2* tw2, const float2* tw, int tid, int nthr) {
     fill_tw2_128h(tw4, tw2, tw, tid, nthr);
   }
   template <bool INV>
-  __device__ static void fft(c2x (&x)[E], float4* buf, const float4*, const float2* tw2, int l, const float4 (&w1)[8]) {
+  __device__ __forceinline__ static void fft(c2x (&x)[E], float4* buf, const float4*, const float2* tw2, int l, const float4 (&w1)[8]) {
     reg_fft2_128h<INV>(x, buf, tw2, l, w1);
   }
 };
@@ -64,14 +64,14 @@ struct XMT<256> {   // a whole warp per row: three stages, 8 x 8 x 4 (reg_fft2_2
   // slot of out[l + 32 j]: j = h + 2 q in slot h*4 + q
   __host__ __device__ static constexpr int jslot(int j) { return (j % 2) * 4 + j / 2; }
   __host__ __device__ static constexpr int kslot(int i) { return jslot(i); }
-  __device__ static int kmode(int l, int i) { return l + 32 * i; }
+  __device__ __forceinline__ static int kmode(int l, int i) { return l + 32 * i; }
   __host__ __device__ static constexpr int pos(int s) { return s / 4 + 2 * (s % 4); }
   __host__ __device__ static constexpr int partner(int i, bool lane0) { return jslot(lane0 ? (8 - i) % 8 : 7 - i); }
-  __device__ static void fill(float4* tw4, float2* tw2, const float2* tw, int tid, int nthr) {
+  __device__ __forceinline__ static void fill(float4* tw4, float2* tw2, const float2* tw, int tid, int nthr) {
     fill_tw2_256w(tw4, tw2, tw, tid, nthr);
   }
   template <bool INV>
-  __device__ static void fft(c2x (&x)[E], float4* buf, const float4* tw4, const float2* tw2, int l,
+  __device__ __forceinline__ static void fft(c2x (&x)[E], float4* buf, const float4* tw4, const float2* tw2, int l,
                              const float4 (&w1)[8]) {
     reg_fft2_256w<INV>(x, buf, tw4, tw2, l, w1);
   }
@@ -85,14 +85,14 @@ struct XMT<512> {   // a whole warp per row: 16 points per lane (reg_fft2_512w)
   // slot of out[l + 32 j]: j = i + 4 q in slot i*4 + q
   __host__ __device__ static constexpr int jslot(int j) { return (j % 4) * 4 + j / 4; }
   __host__ __device__ static constexpr int kslot(int i) { return jslot(i); }
-  __device__ static int kmode(int l, int i) { return l + 32 * i; }
+  __device__ __forceinline__ static int kmode(int l, int i) { return l + 32 * i; }
   __host__ __device__ static constexpr int pos(int s) { return s / 4 + 4 * (s % 4); }
   __host__ __device__ static constexpr int partner(int i, bool lane0) { return jslot(lane0 ? (16 - i) % 16 : 15 - i); }
-  __device__ static void fill(float4* tw4, float2* tw2, const float2* tw, int tid, int nthr) {
+  __device__ __forceinline__ static void fill(float4* tw4, float2* tw2, const float2* tw, int tid, int nthr) {
     fill_tw2_512w(tw4, tw2, tw, tid, nthr);
   }
   template <bool INV>
-  __device__ static void fft(c2x (&x)[E], float4* buf, const float4* tw4, const float2* tw2, int l,
+  __device__ __forceinline__ static void fft(c2x (&x)[E], float4* buf, const float4* tw4, const float2* tw2, int l,
                              const float4 (&)[8]) {
     reg_fft2_512w<INV>(x, buf, tw4, tw2, l);
   }
