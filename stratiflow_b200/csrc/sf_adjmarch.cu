@@ -58,6 +58,7 @@ __global__ void __launch_bounds__(AMShape<N1, D3>::WARPS * 32, 1) k_adjmarch(con
   float4* tw4 = reinterpret_cast<float4*>(xsm);
   float2* tw2 = reinterpret_cast<float2*>(xsm + sizeof(float4) * T::TWE);
   T::fill(tw4, tw2, a.tw, threadIdx.x, blockDim.x);
+  chain_begin();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
   const int gw = lane / G, l = lane - gw * G;
   __builtin_assume(l >= 0 && l < G);
@@ -380,14 +381,14 @@ static void adjmarch_launch(const StageArgs& a, cudaStream_t st) {
   const Geo& g = a.g;
   const int nsm = sm_count();
   if (D3) {
-    k_adjmarch<N1, D3><<<nsm, X::WARPS * 32, X::smem(X::WARPS), st>>>(a, 0);
+    launch_chained(k_adjmarch<N1, D3>, dim3(nsm), X::WARPS * 32, X::smem(X::WARPS), st, a.chained, a, 0);
     return;
   }
   const long long room = (long long)nsm * X::WARPS * X::W;   // 2D: as k_xmarch's segments
   const int seg = (int)(((long long)g.nrun * g.N3 + room - 1) / room);
   const long long warps = ((long long)g.nrun * ((g.N3 + seg - 1) / seg) + X::W - 1) / X::W;
   const int wb = (int)std::min<long long>(X::WARPS, (warps + nsm - 1) / nsm);
-  k_adjmarch<N1, D3><<<(unsigned)((warps + wb - 1) / wb), wb * 32, X::smem(wb), st>>>(a, seg);
+  launch_chained(k_adjmarch<N1, D3>, dim3((unsigned)((warps + wb - 1) / wb)), wb * 32, X::smem(wb), st, a.chained, a, seg);
 }
 
 // the grids whose rows have a march layout of 8 points per lane

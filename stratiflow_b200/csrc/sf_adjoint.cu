@@ -671,6 +671,7 @@ int launch_stage_adjoint(StageArgs a, const float2* below, const float2* above, 
                                                                                   adir);
   a.adir = adir;
   a.adjoint = 1;
+  a.chained = 1;
   if (g.dim3) {
     switch (g.N2) {
       case 16: ify_adj_launch<16>(a, st); break;

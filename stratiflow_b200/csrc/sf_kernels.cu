@@ -94,6 +94,7 @@ __global__ void __launch_bounds__(kYThreads) k_ifft_y2(StageArgs a) {
   const bool act = j1 < g.K1;
   const float2* srcA = a.S + ((size_t)(run * 5 + (p ? 3 : 0)) * g.N3 + j) * g.Pp + j1;
   const float2* srcB = a.S + ((size_t)(run * 5 + (p ? 1 : 2)) * g.N3 + j) * g.Pp + j1;
+  chain_begin();
   c2x x[E];
 #pragma unroll
   for (int e = 0; e < E; e++) {
@@ -139,6 +140,7 @@ __global__ void __launch_bounds__(kYThreads) k_fft_y(StageArgs a) {
   const size_t ps = (size_t)g.N3 * N2 * g.K1;   // one pair's values
   const float4* src = reinterpret_cast<const float4*>(a.mixout) + (size_t)(run * 4 + 2 * p) * ps + (size_t)j * N2 * g.K1 + j1;
   float4* buf = fbuf4 + grp * Y::BUF;
+  chain_begin();
   c2x y[E], x[E];
 #pragma unroll
   for (int e = 0; e < E; e++) {
@@ -1355,14 +1357,14 @@ template <int N2>
 static void ify_launch(const StageArgs& a, int nz, cudaStream_t st) {
   const int nl = a.nlvl > 0 ? a.nlvl : a.g.N3 - a.lvl0;
   if (nz % 4 == 0)   // whole runs: the fields in packed pairs
-    k_ifft_y2<N2><<<dim3(cdiv(a.g.K1, ycols<N2>()), nl, nz / 2), kYThreads, 0, st>>>(a);
+    launch_chained(k_ifft_y2<N2>, dim3(cdiv(a.g.K1, ycols<N2>()), nl, nz / 2), kYThreads, 0, st, a.chained, a);
   else
     k_ifft_y<N2><<<dim3(cdiv(a.g.K1, ycols<N2>()), nl, nz), kYThreads, 0, st>>>(a);
 }
 template <int N2>
 static void fy_launch(const StageArgs& a, cudaStream_t st) {
   const int nl = a.nlvl > 0 ? a.nlvl : a.g.N3 - a.lvl0;
-  k_fft_y<N2><<<dim3(cdiv(a.g.K1, ypcols<N2>()), nl, a.g.nrun * 2), kYThreads, 0, st>>>(a);
+  launch_chained(k_fft_y<N2>, dim3(cdiv(a.g.K1, ypcols<N2>()), nl, a.g.nrun * 2), kYThreads, 0, st, a.chained, a);
 }
 static void launch_ifft_y_z(const StageArgs& a, int nz, cudaStream_t st) {
   switch (a.g.N2) {
@@ -1514,13 +1516,15 @@ static int launch_xy_banded(const StageArgs& a, cudaStream_t st, const XYAux& au
   return 3 * B;
 }
 
-int launch_stage(const StageArgs& a, cudaStream_t st, cudaEvent_t* ev, const XYAux* aux) {
+int launch_stage(const StageArgs& args, cudaStream_t st, cudaEvent_t* ev, const XYAux* aux) {
+  StageArgs a = args;
   const Geo& g = a.g;
   if (g.dim3 && aux && aux->bands > 1 && !ev && !a.tlm) {
     const int n = launch_xy_banded(a, st, *aux);
     launch_z_step(a, st);
     return n + 1;
   }
+  a.chained = !ev;
   int n = 0;
   auto mark = [&]() {
     if (ev) cudaEventRecord(ev[n], st);

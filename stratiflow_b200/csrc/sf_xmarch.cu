@@ -38,6 +38,7 @@ __global__ void __launch_bounds__(XMShape<N1, D3, MODE>::WARPS * 32, 1) k_xmarch
   constexpr int W = XMT<N1>::W;
   extern __shared__ __align__(16) unsigned char xsm[];
   xmarch_tables<N1>(xsm, a.tw);
+  chain_begin();
   __syncthreads();
   const int L = t_hi - t_lo, nwarps = blockDim.x >> 5;
   const long long NW = (long long)gridDim.x * nwarps, wid = (long long)blockIdx.x * nwarps + (threadIdx.x >> 5);
@@ -50,7 +51,7 @@ static void xmarch_launch(const StageArgs& a, int nruns, int t_lo, int t_hi, cud
   using X = XMShape<N1, D3, MODE>;
   const int nsm = sm_count();
   if (D3) {
-    k_xmarch<N1, D3, MODE><<<nsm, X::WARPS * 32, X::smem(X::WARPS), st>>>(a, nruns, t_lo, t_hi, 0);
+    launch_chained(k_xmarch<N1, D3, MODE>, dim3(nsm), X::WARPS * 32, X::smem(X::WARPS), st, a.chained, a, nruns, t_lo, t_hi, 0);
     return;
   }
   // 2D: the shortest segments that all the launch's groups together hold at
@@ -59,7 +60,8 @@ static void xmarch_launch(const StageArgs& a, int nruns, int t_lo, int t_hi, cud
   const int seg = (int)((nruns * L + room - 1) / room);
   const long long warps = (nruns * ((L + seg - 1) / seg) + X::W - 1) / X::W;
   const int wb = (int)std::min<long long>(X::WARPS, (warps + nsm - 1) / nsm);
-  k_xmarch<N1, D3, MODE><<<(unsigned)((warps + wb - 1) / wb), wb * 32, X::smem(wb), st>>>(a, nruns, t_lo, t_hi, seg);
+  launch_chained(k_xmarch<N1, D3, MODE>, dim3((unsigned)((warps + wb - 1) / wb)), wb * 32, X::smem(wb), st, a.chained, a, nruns,
+                 t_lo, t_hi, seg);
 }
 
 // mode 0 nonlinear, 1 frozen base, 2 live base. 3D: every grid whose row has a

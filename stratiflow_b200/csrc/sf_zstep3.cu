@@ -11,6 +11,7 @@ namespace sf {
 // blocks per SM that the registers are held to
 template <int NF, int CQ, int L, int PL, int U, bool SM, bool COL, bool PIPE, int NB>
 __global__ void __launch_bounds__(ZfShape<NF, CQ>::THREADS, NB) k_z_step_f(StageArgs a) {
+  if (!SM || COL) chain_begin();   // else when the tables are filled
   z_step_f_body<NF, CQ, L, PL, U, SM, COL, PIPE>(a, blockIdx.x, blockIdx.z);
 }
 
@@ -89,7 +90,7 @@ bool zstep_f_supported(const Geo& g) { return zf_pick(g, 0) && zf_pick(g, 16); }
 
 int launch_z_step_f(const StageArgs& a, cudaStream_t st) {
   const ZfKernel& k = *zf_pick(a.g, a.zchunks);
-  k.fn<<<dim3((a.g.P + kFM - 1) / kFM, 1, a.g.nrun), k.threads, k.smem(a.g.N3), st>>>(a);
+  launch_chained(k.fn, dim3((a.g.P + kFM - 1) / kFM, 1, a.g.nrun), k.threads, k.smem(a.g.N3), st, a.chained, a);
   return 1;
 }
 

@@ -367,6 +367,7 @@ __device__ __forceinline__ void z_step_f_body(const StageArgs& a, const int bx, 
     tab.c = T + 4 * N3;
     tab.dB = dB;
     if (COL) zf_cp_wait();
+    else chain_begin();
     __syncthreads();
   } else {
     tab.n = a.zt1 + a.stage * N3;
