@@ -14,8 +14,8 @@ kernels' launch shapes, which change no result (or only its rounding):
             neighbouring bands' x passes (sf_set_xy_bands; 3D only)
   z_chunks  block size of the z solves, 8 or 16 (sf_set_z_chunks; 0 = the
             launcher's choice from the grid size)
-  xkernel   the 3D nonlinear x pass as level-marching warps (1) or slab
-            blocks (0) (sf_set_xpass_kernel; 3D only)
+  xkernel   the x pass as level-marching warps (1) or slab
+            blocks (0) (sf_set_xpass_kernel; tried in 3D only)
   zkernel   the z pass as k_z_step_f (2, every field of a mode group at once),
             k_z_step (0) or k_z_step_tma (1, inputs brought in by
             tensor-map copies; applies with 8 z-chunks) (sf_set_z_kernel)

@@ -15,8 +15,8 @@
 // runs out sets *err and skips its item. The host clears the counters before
 // each step.
 //
-// 64 runs, N1 in {64, 128, 256}, N3 in {128, 256, 384}, per stage: 162 us (x items
-// 77, z items 99, each alone in a launch); with slab x items and one field
+// 64 runs, N1 in {64, 128, 256}, N3 in {128, 256, 384}, per stage: 153 us (x items
+// 70, z items 93, each alone in a launch); with slab x items and one field
 // after the other in the z items, two blocks of 8 warps per SM, 243 (135, 108).
 #include <algorithm>
 

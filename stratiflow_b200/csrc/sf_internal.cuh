@@ -91,7 +91,7 @@ struct StageArgs {
   int lvl0, nlvl, xcol0, xcols;
   int zchunks;      // z chunks per block of the z solves (8 or 16; 0: chosen by the launcher)
   int xgroups;      // lane groups per x-pass block (0: chosen by the launcher)
-  int xkernel;      // 3D nonlinear x pass: 1 level-marching lane groups (k_xmarch), 0 slab blocks (k_xpass)
+  int xkernel;      // x pass: 1 level-marching lane groups (k_xmarch) where they pay, 0 slab blocks (k_xpass)
   int zkernel;      // z pass: 0 k_z_step, 1 k_z_step_tma (inputs by the tensor-memory accelerator),
                     // 2 k_z_step_f (every field of a mode group at once)
   const void* zmaps;   // host ZMaps of the solver (k_z_step_tma), or null

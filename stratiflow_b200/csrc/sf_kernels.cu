@@ -2,16 +2,18 @@
 //
 // A stage runs as
 //   [3D] k_ifft_y   modal u1,u2,u3,b -> (kx, y) rows          (ModalField::ToNodal, y part)
-//        k_xpass    per (y row, slab of z levels): c2r along x, the nodal
-//                   products of BuildRHS / BuildRHSLinear, r2c along x,
-//                   1/(N1 N2), 2/3 truncation and the z stencils and
-//                   x-derivatives that follow each product
+//        k_xmarch   (sf_xmarch.cu; small 2D launches: k_xpass, per y row and
+//                   slab of z levels): c2r along x, the nodal products of
+//                   BuildRHS / BuildRHSLinear, r2c along x, 1/(N1 N2), 2/3
+//                   truncation and the z stencils and x-derivatives that
+//                   follow each product
 //   [3D] k_fft_y    (kx, y) -> (kx, ky), y-derivatives, sum into r
-//        k_z_step   per group of 16 modes: for every field ExplicitRK + linear
-//                   buoyancy terms + FinishRHS + CrankNicolson right-hand side +
-//                   Thomas solve, then the divergence, Laplacian solve,
-//                   projection and p update (k_z_proj_chunked alone serves
-//                   RemoveDivergence outside a step)
+//        k_z_step_f (sf_zstep3.cu; also k_z_step here and sf_zstep*.cu) per group
+//                   of modes: for every field ExplicitRK + linear buoyancy terms
+//                   + FinishRHS + CrankNicolson right-hand side + Thomas solve,
+//                   then the divergence, Laplacian solve, projection and p
+//                   update (k_z_proj_chunked alone serves RemoveDivergence
+//                   outside a step)
 // Every kernel touches only kept (dealiased) modes, which is all the reference's
 // ModalField arithmetic touches (Field.h:1129-1166).
 

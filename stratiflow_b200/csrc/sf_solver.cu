@@ -61,7 +61,7 @@ struct sf_solver {
   int xy_bands = 1;              // level bands of the 3D x-y pass (sf_set_xy_bands)
   int zchunks = 0;               // z chunks per z-solve block (sf_set_z_chunks)
   int xgroups = 0;               // lane groups per x-pass block (sf_set_xpass_groups)
-  int xkernel = 1;               // 3D nonlinear x pass: 1 level-marching, 0 slab blocks (sf_set_xpass_kernel)
+  int xkernel = 1;               // x pass: 1 level-marching, 0 slab blocks (sf_set_xpass_kernel)
   int zkernel = 2;               // z pass: 2 k_z_step_f (default), 0 k_z_step, 1 k_z_step_tma (sf_set_z_kernel)
   ZMaps* zmaps = nullptr;        // tensor maps of k_z_step_tma's inputs (null: not supported here)
   int* zerr = nullptr;           // set on the device by a k_z_step_tma wait that ran out

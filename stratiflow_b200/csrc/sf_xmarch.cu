@@ -68,11 +68,13 @@ static void xmarch_launch(const StageArgs& a, int nruns, int t_lo, int t_hi, cud
 // shape here. 2D, where the slab kernel's blocks spread a few levels over more
 // SMs: from 2^18 points of the launch's runs (mode 1, whose slabs copy the
 // base's rows as well, always). Measured per launch (us), slab and march:
-//   2D nonlinear  1 x 128x128 12.7 13.5; 2 x 256x256 12.7 14.1; 4 x 256x256 16.8 14.7; 6 x 512x388 57.2 39.0;
-//                 32 x 256x256 59.7 42.8; 8 x 64x128 11.7 12.9; 16 x 64x256 21.0 15.0
-//   2D frozen     1 x 64x64 12.6 12.6; 1 x 128x128 16.0 14.0; 4 x 256x256 28.9 16.7
-//   2D live base  1 + 2 x 512x200 52.6 57.7; 1 + 4 x 256x256 40.3 29.8
-//   3D            2 x 128x64x180 130 69; frozen 2 x 128x64x192 256 101; frozen 256x64x128 175 73
+//   2D nonlinear  1 x 128x128 12.7 13.5 (1); 2 x 256x256 12.7 14.1 (1); 8 x 64x128 11.7 12.9 (1); 4 x 256x256 17.9 15.8;
+//                 16 x 64x256 20.9 14.0; 6 x 512x388 57.6 36.5; 32 x 256x256 61.0 37.8
+//   2D frozen     1 x 64x64 13.5 13.2; 1 x 128x128 15.9 13.8; 4 x 256x256 29.0 17.8
+//   2D live base  1 + 2 x 512x200 55.0 54.8; 1 + 4 x 256x256 40.6 29.9
+//   3D            2 x 128x64x180 131 58; frozen 2 x 128x64x192 258 95; frozen 256x64x128 172 68
+// (1) before the march kept its carried values in registers, which takes a
+// tenth off it.
 bool xmarch_supported(const StageArgs& a, int mode, int nruns) {
   const Geo& g = a.g;
   if (a.adjoint) return false;
