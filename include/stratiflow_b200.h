@@ -222,7 +222,7 @@ int sf_set_xpass_groups(sf_solver* s, int groups);
  * fields or products per packed FP32 instruction; kind 0 as blocks over slabs
  * of levels. The results agree to rounding (the z stencils' terms are summed
  * in another order). 3D grids with N1 other than 64, 128 or 256, small 2D
- * launches (under 2^18 points, except the frozen-base step) and the 2D adjoint
+ * launches (under 2^17 points, 2^13 at N1 = 128, except the frozen-base step) and the 2D adjoint
  * outside N1 = 32 .. 256 always take kind 0. */
 int sf_set_xpass_kernel(sf_solver* s, int kind);
 

@@ -104,7 +104,7 @@ struct StageArgs {
 // before it are filled, and they wait (chain_begin) until its results are
 // visible. Hides the kernels' launch latency where it counts: 64x32x64, four
 // steps 275 -> 264 us; adjoint step at 128x64x128 389 -> 368; 64x64 in 2D 46 ->
-// 45; larger grids do not notice. Letting the next kernel's blocks in earlier,
+// 44; larger grids do not notice. Letting the next kernel's blocks in earlier,
 // while the last wave still runs, costs more than it gives (302 us, and 1690
 // for 1564 at 256x128x384): they hold places that work would be spread over. In
 // a kernel that was launched in the ordinary way chain_begin does nothing.

@@ -654,6 +654,7 @@ __device__ __forceinline__ void xpass_body(const StageArgs& a, int S, int iters,
 
 template <int N1, bool LINEAR>
 __global__ void __launch_bounds__(kXMaxThreads) k_xpass(StageArgs a, int S, int iters) {
+  chain_begin();
   xpass_body<N1, LINEAR>(a, S, iters, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
@@ -1289,7 +1290,7 @@ static void xpass_launch(const StageArgs& a, int nruns, cudaStream_t st) {
   const int ncol = (int)cdiv(g.N3, x.S * x.iters);
   const int cols = a.xcols > 0 ? a.xcols : ncol - a.xcol0;
   dim3 grid(cols, g.N2, nruns);
-  k_xpass<N1, LIN><<<grid, x.threads, x.bytes, st>>>(a, x.S, x.iters);
+  launch_chained(k_xpass<N1, LIN>, grid, x.threads, x.bytes, st, a.chained, a, x.S, x.iters);
 }
 
 template <int N1>

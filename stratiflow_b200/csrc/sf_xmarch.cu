@@ -65,22 +65,24 @@ static void xmarch_launch(const StageArgs& a, int nruns, int t_lo, int t_hi, cud
 }
 
 // mode 0 nonlinear, 1 frozen base, 2 live base. 3D: every grid whose row has a
-// shape here. 2D, where the slab kernel's blocks spread a few levels over more
-// SMs: from 2^18 points of the launch's runs (mode 1, whose slabs copy the
-// base's rows as well, always). Measured per launch (us), slab and march:
-//   2D nonlinear  1 x 128x128 12.7 13.5 (1); 2 x 256x256 12.7 14.1 (1); 8 x 64x128 11.7 12.9 (1); 4 x 256x256 17.9 15.8;
-//                 16 x 64x256 20.9 14.0; 6 x 512x388 57.6 36.5; 32 x 256x256 61.0 37.8
+// shape here. 2D: where the slab kernel's blocks do not spread a few levels over
+// more SMs, from 2^17 points of the launch's runs, 2^13 at N1 = 128, whose rows
+// march two to a warp at 8 points a lane; always in mode 1, whose slabs copy the base's
+// rows as well. Measured, a whole step (us), slab and march:
+//   N1 = 128      64 levels 37.8 36.9; 128 levels 47.1 45.1; 4 x 256 76.7 72.4; 1 + 2 tangents, 128 levels 83.4 73.8
+//   others        64x64 32.8 34.9; 256x64 36.9 38.9; 64x64 x 4 33.8 36.9; 256x128 47.1 49.5; 64x128 x 8 45.1 46.0;
+//                 256x256 x 2 75.8 75.8; 256x256 x 3 79.9 80.7; 512x388 110.9 107.6; 32x256 x 16 71.7 69.7
+// and per launch:
+//   2D nonlinear  4 x 256x256 17.9 15.8; 16 x 64x256 20.9 14.0; 6 x 512x388 57.6 36.5; 32 x 256x256 61.0 37.8
 //   2D frozen     1 x 64x64 13.5 13.2; 1 x 128x128 15.9 13.8; 4 x 256x256 29.0 17.8
 //   2D live base  1 + 2 x 512x200 55.0 54.8; 1 + 4 x 256x256 40.6 29.9
 //   3D            2 x 128x64x180 131 58; frozen 2 x 128x64x192 258 95; frozen 256x64x128 172 68
-// (1) before the march kept its carried values in registers, which takes a
-// tenth off it.
 bool xmarch_supported(const StageArgs& a, int mode, int nruns) {
   const Geo& g = a.g;
   if (a.adjoint) return false;
   const int N1 = g.N1;
   if (g.dim3) return (N1 == 64 || N1 == 128 || N1 == 256) && g.N2 % 4 == 0;
-  return N1 <= 512 && (mode == 1 || (long long)N1 * g.N3 * nruns >= (1 << 18));
+  return N1 <= 512 && (mode == 1 || (long long)N1 * g.N3 * nruns >= (N1 == 128 ? 1 << 13 : 1 << 17));
 }
 
 template <int N1, bool D3>
