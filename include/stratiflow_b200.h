@@ -373,7 +373,7 @@ int sf_net_get_params(sf_net* n, float* host);
 int sf_net_set_params(sf_net* n, const float* host);
 /* y[batch][Z][Cout] = net(x[batch][Z][Cin]); discards the training data */
 int sf_net_forward(sf_net* n, const float* x, int batch, float* y);
-/* uploads a training set: inputs x[batch][Z][Cin], targets [batch][Z][Cout] */
+/* uploads a training set: inputs x[batch][Z][Cin], targets [batch][Z][Cout]; both have been read on return */
 int sf_net_set_data(sf_net* n, const float* x, const float* target, int batch);
 /* mean-square loss over the training set and its gradient (parameter layout) */
 int sf_net_gradient(sf_net* n, float* grad, double* loss);

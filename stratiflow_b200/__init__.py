@@ -740,7 +740,6 @@ class Net:
         target = np.ascontiguousarray(target, dtype=np.float32)
         B = x.shape[0]
         assert x.shape == (B, self.Z, self.channels[0]) and target.shape == (B, self.Z, self.channels[-1])
-        self._data = (x, target)   # the host arrays outlive the asynchronous upload
         _check(load_library().sf_net_set_data(self._h, _fptr(x), _fptr(target), B))
 
     def gradient(self):

@@ -671,6 +671,8 @@ int sf_net_set_data(sf_net* n, const float* x, const float* target, int batch) {
   if (rc) return rc;
   NCK(cudaMemcpyAsync(n->tgt, target, sizeof(float) * batch * n->Z * n->ch[n->nl], cudaMemcpyHostToDevice,
                       n->st));
+  // the caller may change x and target from here on, page-locked or not
+  NCK(cudaStreamSynchronize(n->st));
   n->nb_data = batch;
   return SF_OK;
 }
