@@ -6,7 +6,6 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
-#include <mutex>
 #include <string>
 #include <vector>
 
@@ -312,17 +311,6 @@ const float2* sf_solver_tw(const sf_solver* s) { return s->tw; }
 const float* sf_solver_ubar(const sf_solver* s, int run) { return s->Ubar + (size_t)run * s->g.N3; }
 void sf_solver_count_launches(sf_solver* s, int n) { s->launches += n; }
 
-// the kernels' shared-memory limits, set once per device (the current one)
-static bool kernels_ready(int device) {
-  static std::mutex mu;
-  static std::vector<int> done;
-  std::lock_guard<std::mutex> lock(mu);
-  if (std::find(done.begin(), done.end(), device) != done.end()) return true;
-  if (prepare_kernels() != 0 || prepare_adjoint_kernels() != 0) return false;
-  done.push_back(device);
-  return true;
-}
-
 extern "C" {
 
 const char* sf_last_error(void) { return g_err.c_str(); }
@@ -367,7 +355,9 @@ int sf_create(const sf_grid* grid, const sf_flow* flow, double dt, int device, s
     }                                                                                              \
   } while (0)
 
-  if (!kernels_ready(device)) return cleanup_fail(fail(SF_ECUDA, "cudaFuncSetAttribute failed"));
+  // on each creation: the limits go with the device's context, which a reset of the device replaces
+  if (prepare_kernels() != 0 || prepare_adjoint_kernels() != 0)
+    return cleanup_fail(fail(SF_ECUDA, "cudaFuncSetAttribute failed"));
   CKC(cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking));
   if (g.dim3) {
     CKC(cudaStreamCreateWithFlags(&s->xy.y1, cudaStreamNonBlocking));
