@@ -130,12 +130,13 @@ def _fptr(a: np.ndarray):
 
 
 class _ResultBuffers:
-    """Page-locked host memory for large results, so that they arrive by one
-    direct copy instead of through the driver's staging and the first touch of
-    new pages (10.5 MB of a predictor gradient: 0.2 ms against 1.3). An array
-    made here is the caller's; its memory comes back when the last view of it
-    is gone. At most LIMIT bytes are held, in use or waiting; past that, and
-    for results under SMALL bytes, the array is ordinary memory."""
+    """Host memory for large results, into which they arrive by one direct copy
+    instead of through the driver's staging and the first touch of new pages
+    (10.5 MB of a predictor gradient: 0.2 ms against 1.3). An array made here
+    is the caller's, and ordinary memory to everything but that copy
+    (sf_host_alloc); its memory comes back when the last view of it is gone.
+    At most LIMIT bytes are held, in use or waiting; past that, and for
+    results under SMALL bytes, the array is ordinary memory of its own."""
     LIMIT, SMALL = 64 << 20, 1 << 18
 
     def __init__(self):

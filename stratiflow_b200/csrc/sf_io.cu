@@ -204,18 +204,4 @@ int sf_velocity_maxima(sf_solver* s, int run, double* out) {
   return SF_OK;
 }
 
-int sf_host_alloc(size_t bytes, void** ptr) {
-  if (!ptr || bytes == 0) return iofail(SF_EINVAL, "bad argument");
-  const cudaError_t e = cudaHostAlloc(ptr, bytes, cudaHostAllocPortable);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    return iofail(SF_ENOMEM, std::string("cudaHostAlloc: ") + cudaGetErrorString(e));
-  }
-  return SF_OK;
-}
-int sf_host_free(void* ptr) {
-  if (ptr) ICK(cudaFreeHost(ptr));
-  return SF_OK;
-}
-
 }  // extern "C"

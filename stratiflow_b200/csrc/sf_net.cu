@@ -28,6 +28,7 @@
 #include "../../include/stratiflow_b200.h"
 
 extern void sf_set_error_message(const std::string& msg);
+extern void* sf_host_dma(void* p);
 
 namespace {
 
@@ -661,7 +662,7 @@ int sf_net_forward(sf_net* n, const float* x, int batch, float* y) {
   if (!rc) rc = forward(n, batch, true);
   if (rc) return rc;
   n->nb_data = 0;   // act[0] no longer holds the training inputs
-  NCK(cudaMemcpyAsync(y, n->out, sizeof(float) * batch * n->Z * n->ch[n->nl], cudaMemcpyDeviceToHost, n->st));
+  NCK(cudaMemcpyAsync(sf_host_dma(y), n->out, sizeof(float) * batch * n->Z * n->ch[n->nl], cudaMemcpyDeviceToHost, n->st));
   return net_status(n);
 }
 
@@ -682,7 +683,7 @@ int sf_net_gradient(sf_net* n, float* grad, double* loss) {
   int rc = forward(n, n->nb_data, true);
   if (!rc) rc = backward(n, n->nb_data);
   if (rc) return rc;
-  if (grad) NCK(cudaMemcpyAsync(grad, n->gr, sizeof(float) * n->nparam, cudaMemcpyDeviceToHost, n->st));
+  if (grad) NCK(cudaMemcpyAsync(sf_host_dma(grad), n->gr, sizeof(float) * n->nparam, cudaMemcpyDeviceToHost, n->st));
   if (loss) NCK(cudaMemcpyAsync(loss, n->loss, sizeof(double), cudaMemcpyDeviceToHost, n->st));
   return net_status(n);
 }

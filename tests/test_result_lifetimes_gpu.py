@@ -34,3 +34,60 @@ def test_set_data_has_read_its_arrays_when_it_returns():
     y -= 1.0
     _, loss = n.gradient()
     assert abs(loss - 1.0) < 1e-4
+
+
+def test_a_result_can_be_changed_or_dropped_under_a_queued_copy():
+    import torch
+    n, x = _net()
+    y = n.forward(x)
+    want = y.copy()
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        _delay()
+        d = torch.from_numpy(y).to("cuda", non_blocking=True)
+    y[:] = 0.0
+    side.synchronize()
+    assert torch.equal(d.cpu(), torch.from_numpy(want))
+    y = n.forward(x)
+    with torch.cuda.stream(side):
+        _delay()
+        d = torch.from_numpy(y).to("cuda", non_blocking=True)
+    del y
+    n.forward(-x)                  # takes the buffer that came back
+    side.synchronize()
+    assert torch.equal(d.cpu(), torch.from_numpy(want))
+
+
+RESET = """
+import ctypes, os
+import numpy as np
+import stratiflow_b200 as sf
+import nvidia.cuda_runtime
+rng = np.random.default_rng(4)
+
+def gradient():
+    n = sf.Net([64, 256, 512], 64, 4, seed=3)
+    n.set_params(w)
+    n.set_data(x, t)
+    return n.gradient()[0]
+
+w = rng.normal(0, 0.05, 64 * 5 * 256 + 256 + 256 * 5 * 512 + 512).astype(np.float32)
+x, t = (rng.normal(0, 1, (4, 64, c)).astype(np.float32) for c in (64, 512))
+a, b = gradient(), gradient()
+want = a.copy()
+del b                              # its buffer waits in the pool
+rt = ctypes.CDLL(os.path.join(list(nvidia.cuda_runtime.__path__)[0], "lib", "libcudart.so.12"))
+assert rt.cudaDeviceReset() == 0
+assert np.array_equal(a, want)
+assert np.array_equal(gradient(), want)
+print("same")
+"""
+
+
+def test_results_outlive_a_reset_of_the_device():
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", RESET], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip() == "same", r.stdout + r.stderr
