@@ -152,12 +152,15 @@ class _ResultBuffers:
                 self.free.setdefault(n, []).append(ptr)
             if self.free.get(nbytes):
                 return self.free[nbytes].pop()
+            waiting = sum(size * len(ptrs) for size, ptrs in self.free.items())
+            if self.held - waiting + nbytes > self.LIMIT:   # not even without the waiting buffers
+                return None
             for size, ptrs in list(self.free.items()):   # buffers of other sizes make room
                 while ptrs and self.held + nbytes > self.LIMIT:
                     load_library().sf_host_free(C.c_void_p(ptrs.pop()))
                     self.held -= size
             p = C.c_void_p()
-            if self.held + nbytes > self.LIMIT or load_library().sf_host_alloc(nbytes, C.byref(p)) != 0:
+            if load_library().sf_host_alloc(nbytes, C.byref(p)) != 0:
                 return None
             self.held += nbytes
             return p.value
