@@ -24,11 +24,14 @@ The search is coordinate descent from the launchers' defaults: each setting
 in turn takes every candidate value with the others held, and a value
 replaces the current one only if it is faster by more than the noise margin.
 Plans are cached in memory and in a JSON file (SF_PLAN_CACHE, default
-~/.cache/stratiflow_b200/plans.json) keyed by device name, grid, run count and
-step kind.
+~/.cache/stratiflow_b200/plans.json) keyed by device name, kernels, grid, run
+count and step kind: a plan is a comparison of the kernels it was timed on, and
+says nothing of others that its settings may choose between later.
 """
 from __future__ import annotations
 
+import functools
+import hashlib
 import json
 import os
 import time
@@ -92,8 +95,29 @@ def cache_path() -> str:
                           os.path.join(os.path.expanduser("~"), ".cache", "stratiflow_b200", "plans.json"))
 
 
+HERE = os.path.dirname(os.path.abspath(__file__))
+CSRC = os.path.join(HERE, "csrc")
+
+
+@functools.lru_cache(maxsize=None)
+def kernels_version(csrc: str | None = None) -> str:
+    """Names the kernels: a digest of their sources (1 ms, once a process), or
+    of the library where it was installed without them."""
+    csrc = csrc or CSRC
+    if os.path.isdir(csrc):
+        files = [os.path.join(csrc, f) for f in sorted(os.listdir(csrc))]
+    else:
+        files = [os.path.join(HERE, "libstratiflow_b200.so")]
+    h = hashlib.sha256()
+    for f in files:
+        if os.path.isfile(f):
+            with open(f, "rb") as src:
+                h.update(os.path.basename(f).encode() + b"\0" + src.read() + b"\0")
+    return h.hexdigest()[:12]
+
+
 def plan_key(device: str, N1: int, N2: int, N3: int, nrun: int, mode: str) -> str:
-    return f"{device}|{N1}x{N2}x{N3}|runs {nrun}|{mode}"
+    return f"{device}|kernels {kernels_version()}|{N1}x{N2}x{N3}|runs {nrun}|{mode}"
 
 
 def load_cache(path: str | None = None) -> Dict[str, dict]:
