@@ -251,7 +251,7 @@ int sf_dot(sf_solver* sa, int run_a, sf_solver* sb, int run_b, double* out);
  * sf_step_linear (linear != 0). Slot order is that of sf_profile_names. */
 int sf_profile_step(sf_solver* s, int nsteps, int linear, int cap, double* ms, int* nslots);
 
-/* comma-separated kernel names of the profile slots */
+/* comma-separated kernel names of the slots of the last sf_profile_step (before any: of a nonlinear step) */
 int sf_profile_names(sf_solver* s, char* buf, size_t len);
 
 /* RemoveDivergence(pressure_multiplier) for callers that cannot allocate

@@ -64,6 +64,7 @@ struct sf_solver {
   int zkernel = 2;               // z pass: 2 k_z_step_f (default), 0 k_z_step, 1 k_z_step_tma (sf_set_z_kernel)
   ZMaps* zmaps = nullptr;        // tensor maps of k_z_step_tma's inputs (null: not supported here)
   int* zerr = nullptr;           // set on the device by a k_z_step_tma wait that ran out
+  bool profiled_linear = false;  // the last sf_profile_step took linear steps (sf_profile_names)
   cudaGraphExec_t graph[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};   // [linear][parity]
   long long launches = 0;
   long long launches_per_step[2] = {0, 0};
@@ -785,6 +786,7 @@ int sf_profile_step(sf_solver* s, int nsteps, int linear, int cap, double* ms, i
   if (linear && !s->base_set) return fail(SF_ESTATE, "linear profile needs sf_set_base first");
   const int per = stage_kernel_count(s->g), n = 3 * per;
   if (cap < n) return fail(SF_EINVAL, "ms buffer too small");
+  s->profiled_linear = linear != 0;
   std::vector<cudaEvent_t> ev(n + 1);
   for (auto& e : ev) CK(cudaEventCreate(&e));
   std::vector<double> acc(n, 0.0);
@@ -812,10 +814,9 @@ int sf_profile_step(sf_solver* s, int nsteps, int linear, int cap, double* ms, i
 int sf_profile_names(sf_solver* s, char* buf, size_t len) {
   if (!s || !buf || len == 0) return fail(SF_EINVAL, "bad argument");
   std::string out;
-  // the x pass runs as k_xmarch where the solver takes it
-  const bool march = s->xkernel == 1 && xmarch_supported(stage_args(s, 0, s->cur, false), s->tlm ? 2 : 0, s->g.nrun - s->tlm);
-  // and the z pass as k_z_step_tma
-  const StageArgs a0 = stage_args(s, 0, s->cur, false);
+  // the x pass of the profiled step (a tangent batch's: of its tangents) runs as k_xmarch where the solver takes it
+  const StageArgs a0 = stage_args(s, 0, s->cur, s->profiled_linear);
+  const bool march = s->xkernel == 1 && xmarch_supported(a0, s->tlm ? 2 : (s->profiled_linear ? 1 : 0), s->g.nrun - s->tlm);
   const char* zname = z_step_takes_c(a0) ? (zstep_f_supported(a0.g) ? "k_z_step_f" : "k_z_step_c") : (z_step_takes_tma(a0) ? "k_z_step_tma" : "k_z_step");
   for (int k = 0; k < 3; k++)
     for (int i = 0; i < stage_kernel_count(s->g); i++) {
