@@ -202,11 +202,17 @@ def kernel_bytes(s, name):
         return (4 * M + 8 * M) if s.dim3 else (3 * S + 3 * S)
     if name == "k_fft_y":
         return 8 * M + 4 * S
-    if name in ("k_z_step", "k_z_step_tma", "k_z_step_c", "k_z_step_f"):
+    if name in ("k_z_step", "k_z_step_tma", "k_z_step_c"):
         # in: u (nf fields), p, r_nl, r_old, and the per-mode factors 1/den_j
         # (float, half a complex field) of the velocity, u3, b and Laplacian
         # systems; out: u, p and r_old for the next stage
         return (3 * nf + 1 + 2) * S + (2 * nf + 1) * S
+    if name == "k_z_step_f":
+        # averaged over the three stages: the buffers of r take turns, so r_old
+        # is read in the second and third stage and written in none; out: u, p
+        # and, in the first two stages, the completed r of u3 and b (3D 18, 22
+        # and 20 S, 2D 15, 18 and 16 S)
+        return ((6 * nf + 2 * nf + 3 * 3) * S + (3 * (nf + 1) + 2 * 2) * S) / 3.0
     return 0
 
 
