@@ -284,8 +284,10 @@ int sf_remove_divergence_noalloc(const sf_grid* grid, const sf_flow* flow, doubl
  * members' own queued work first and returns without waiting for the steps:
  * call sf_ensemble_synchronize before using a member again. Members must not
  * be stepped on their own in between (sf_ensemble_step then reports
- * SF_ESTATE if their state parities differ). The member handles belong to
- * the ensemble: sf_ensemble_destroy frees them. */
+ * SF_ESTATE if their state parities differ). Of a member's launch settings
+ * its z kernel holds here (sf_set_z_kernel; 0 and 1 both take k_z_step's
+ * solves). The member handles belong to the ensemble: sf_ensemble_destroy
+ * frees them. */
 typedef struct sf_ensemble sf_ensemble;
 int sf_ensemble_create(int nrun, const sf_grid* grids, const sf_flow* flows, const double* dt, int device,
                        sf_ensemble** out);

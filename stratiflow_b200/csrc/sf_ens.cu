@@ -5,7 +5,9 @@
 // all x-pass items first (largest members first), then all z items. An x item
 // is 12 warps' worth of a member's level segments, marched by xmarch_rows
 // (sf_xmarch.cuh); a z item is 8 modes of a member, by z_step_f_body
-// (sf_zstep_f.cuh) whose 12 warps are 3 fields x 4. A z item of member r
+// (sf_zstep_f.cuh) whose 12 warps are 3 fields x 4; a member whose own z kernel
+// is k_z_step or k_z_step_tma has z_step_body instead (sf_zstep_k.cuh, 16 modes
+// by 12 chunks, at every other item). A z item of member r
 // starts once member r's x items have all finished (counters[1 + r] reaches
 // xneed[r]). A block claims its next item as it starts the current one, so
 // the claim's latency hides behind the work; every wait still ends: an item
@@ -22,6 +24,7 @@
 
 #include "sf_xmarch.cuh"
 #include "sf_zstep_f.cuh"
+#include "sf_zstep_k.cuh"
 
 namespace sf {
 
@@ -106,6 +109,13 @@ __global__ void __launch_bounds__(kEnsThreads, 1) k_ens_stage(const StageArgs* _
         __threadfence();   // this item's r rows, before it counts as done
         atomicAdd(&counters[1 + it.run], 1);
       }
+    } else if (ok && sa.zkernel != 2) {   // the member asks for the other z kernels' solves
+      tables = 0;
+      const int N3 = sa.g.N3, per = N3 <= kEnsFusedN3 ? 2 : 1;   // items per 16 modes
+      if (it.x % per == 0) {
+        if ((N3 + kEnsWarps - 1) / kEnsWarps >= 48) z_step_body<kEnsWarps, true>(sa, it.x / per, 0);
+        else z_step_body<kEnsWarps, false>(sa, it.x / per, 0);
+      }
     } else if (ok) {   // the shapes of k_z_step_f that 12 warps make (sf_zstep3.cu), else k_z_step_c's
       tables = 0;
       const int N3 = sa.g.N3;
@@ -154,7 +164,8 @@ size_t ensemble_smem(int N1, int N3) {
   }
   const size_t z = N3 > kEnsFusedN3 ? zc_smem_bytes<2 * kEnsWarps>(N3)
                                     : ZfShape<3, 4>::smem(N3, N3 > 64, N3 > 64);
-  return std::max(x, z);
+  const size_t k = sizeof(float) * ((size_t)N3 * 32 + 3 * kEnsWarps * 32);   // z_step_body
+  return std::max(x, std::max(z, k));
 }
 
 int launch_ens_stage(const StageArgs* args, const EnsItem* xitems, int nx, const EnsItem* zitems, int nz,

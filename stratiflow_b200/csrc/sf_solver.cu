@@ -1127,7 +1127,8 @@ int sf_ensemble_step(sf_ensemble* e, int nsteps) {
       for (int r = 0; r < R; r++) {
         StageArgs a;
         std::memset(&a, 0, sizeof(a));   // the padding too: the copies are compared as bytes
-        a = stage_args(e->members[r], k, cur, false, e->members[r]->g.N3 <= kEnsFusedN3);
+        a = stage_args(e->members[r], k, cur, false,
+                       e->members[r]->zkernel == 2 && e->members[r]->g.N3 <= kEnsFusedN3);
         StageArgs& h = e->h_args[((size_t)p * 3 + k) * R + r];
         changed = changed || std::memcmp(&h, &a, sizeof(a)) != 0;
         std::memcpy(&h, &a, sizeof(a));

@@ -1,5 +1,5 @@
 // k_z_step_c: the z pass with one lane per complex mode (the device code is
-// in sf_zstep_c.cuh, which the ensemble kernels of sf_kernels.cu share).
+// in sf_zstep_c.cuh, which the ensembles' stage kernel, sf_ens.cu, shares).
 // CC z-chunks per block, two per warp: 16 (8 warps, 3 blocks per SM) by
 // default, 32 (16 warps, one block per SM) for grids whose blocks leave SMs
 // idle, as k_z_step takes 16 warps there.
