@@ -72,8 +72,8 @@ struct ConvGemm {
 // The K slices, and the runs of 16 of an instruction within them, go in the
 // order of (tap, channel), one accumulator per tile: a result does not depend
 // on the tiling. Every wait is bounded; one that runs out sets *err, the other
-// waits of the block then give up at once, and the block waits for its copies
-// in flight and frees its tensor memory.
+// waits of the block then give up at once, and the block waits, with the same
+// bound, for its copies and instructions in flight and frees its tensor memory.
 constexpr int TM = 128, TN = 64, TK = 64, kTcThreads = 128, kTcStages = 4, kMaxLayers = 16;
 constexpr int kTcABytes = TM * TK * 2, kTcBBytes = TN * TK * 2, kTcStageBytes = kTcABytes + kTcBBytes;
 // the stages, and room to align the first to the swizzle's 1024-byte period
@@ -135,7 +135,7 @@ __device__ __forceinline__ void conv_tile(const CUtensorMap& mapA, const CUtenso
                                           const int tn, const int m0, int* err) {
   extern __shared__ __align__(128) unsigned char tsm[];
   unsigned char* stage0 = tsm + ((1024 - (smem_u32(tsm) & 1023)) & 1023);
-  __shared__ __align__(8) uint64_t full[kTcStages], empty[kTcStages], done;
+  __shared__ __align__(8) uint64_t full[kTcStages], empty[kTcStages], done, drain;
   __shared__ uint32_t tmem_base;
   __shared__ volatile int failed;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -159,15 +159,17 @@ __device__ __forceinline__ void conv_tile(const CUtensorMap& mapA, const CUtenso
       mbar_init(&empty[s]);
     }
     mbar_init(&done);
+    mbar_init(&drain);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = tmem_base;
+  int kt = 0;   // thread 0: the slices whose copies it has issued
   if (warp == 0) {
     if (lane == 0) {
-      int kt = 0, s = 0, ph = 1;   // ph: the parity of the slot's last use
+      int s = 0, ph = 1;   // ph: the parity of the slot's last use
       for (; kt < nk; kt++, s = s + 1 == ns ? 0 : s + 1, ph ^= s == 0) {
         const int k1 = kt / ks, k0 = (kt - k1 * ks) * TK;
         if (kt >= ns && !mbar_wait(&empty[s], ph, &failed)) {
@@ -192,8 +194,6 @@ __device__ __forceinline__ void conv_tile(const CUtensorMap& mapA, const CUtenso
           tma3(Bt, &mapB, n0, k0 + nb - kPad, k1, &full[s]);
         }
       }
-      if (failed)   // the copies in flight
-        for (int i = kt > ns ? kt - ns : 0; i < kt; i++) mbar_wait(&full[i % ns], (i / ns) & 1, &failed, false);
     }
     __syncwarp();
   } else if (warp == 1) {
@@ -204,6 +204,11 @@ __device__ __forceinline__ void conv_tile(const CUtensorMap& mapA, const CUtenso
         if (!mbar_wait(&full[s], ph, &failed)) {
           failed = 1;
           atomicExch(err, 1);
+          // the instructions issued so far, before their operands and accumulator go
+          asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                           smem_u32(&drain))
+                       : "memory");
+          mbar_wait(&drain, 0, &failed, false);
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;");
@@ -232,6 +237,8 @@ __device__ __forceinline__ void conv_tile(const CUtensorMap& mapA, const CUtenso
     failed = 1;
     atomicExch(err, 1);
   }
+  if (!ok && tid == 0)   // the copies in flight, of slices that no instruction has waited for
+    for (int i = kt > ns ? kt - ns : 0; i < kt; i++) mbar_wait(&full[i % ns], (i / ns) & 1, &failed, false);
   __syncwarp();
   asm volatile("tcgen05.fence::after_thread_sync;");
   if (__all_sync(0xffffffffu, ok)) {
