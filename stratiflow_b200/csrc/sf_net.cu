@@ -129,6 +129,22 @@ __device__ __forceinline__ void tma3(void* dst, const CUtensorMap* map, int x, i
       : "memory");
 }
 
+// A block whose wait ran out: the copies in flight, of slices that no
+// instruction has waited for, and the instructions in flight, before their
+// operands and the accumulator go. Not inlined: out of the way of the loops'
+// code, inside which they cost 5 us of a gradient's 418.
+__device__ __noinline__ void drain_copies(uint64_t* full, int issued, volatile int* failed) {
+  for (int i = issued > kTcStages ? issued - kTcStages : 0; i < issued; i++)
+    mbar_wait(&full[i % kTcStages], (i / kTcStages) & 1, failed, false);
+}
+__device__ __noinline__ void drain_instructions(uint64_t* drain, volatile int* failed, int* err) {
+  *failed = 1;
+  atomicExch(err, 1);
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(drain))
+               : "memory");
+  mbar_wait(drain, 0, failed, false);
+}
+
 // tile (tn, m0) of one GEMM
 template <int MODE>
 __device__ __forceinline__ void conv_tile(const CUtensorMap& mapA, const CUtensorMap& mapB, const ConvGemm& p,
@@ -166,10 +182,10 @@ __device__ __forceinline__ void conv_tile(const CUtensorMap& mapA, const CUtenso
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = tmem_base;
-  int kt = 0;   // thread 0: the slices whose copies it has issued
+  int issued = 0;   // thread 0: the slices whose copies it has issued
   if (warp == 0) {
     if (lane == 0) {
-      int s = 0, ph = 1;   // ph: the parity of the slot's last use
+      int kt = 0, s = 0, ph = 1;   // ph: the parity of the slot's last use
       for (; kt < nk; kt++, s = s + 1 == ns ? 0 : s + 1, ph ^= s == 0) {
         const int k1 = kt / ks, k0 = (kt - k1 * ks) * TK;
         if (kt >= ns && !mbar_wait(&empty[s], ph, &failed)) {
@@ -194,23 +210,15 @@ __device__ __forceinline__ void conv_tile(const CUtensorMap& mapA, const CUtenso
           tma3(Bt, &mapB, n0, k0 + nb - kPad, k1, &full[s]);
         }
       }
+      issued = kt;
     }
     __syncwarp();
   } else if (warp == 1) {
     if (lane == 0) {
       constexpr uint32_t idesc = umma_idesc_bf16(TM, TN, a_mn, b_mn);
-      int s = 0, ph = 0;
-      for (int kt = 0; kt < nk; kt++, s = s + 1 == ns ? 0 : s + 1, ph ^= s == 0) {
-        if (!mbar_wait(&full[s], ph, &failed)) {
-          failed = 1;
-          atomicExch(err, 1);
-          // the instructions issued so far, before their operands and accumulator go
-          asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                           smem_u32(&drain))
-                       : "memory");
-          mbar_wait(&drain, 0, &failed, false);
-          break;
-        }
+      int kt = 0, s = 0, ph = 0;
+      for (; kt < nk; kt++, s = s + 1 == ns ? 0 : s + 1, ph ^= s == 0) {
+        if (!mbar_wait(&full[s], ph, &failed)) break;
         asm volatile("tcgen05.fence::after_thread_sync;");
         const uint32_t a0 = smem_u32(stage0) + s * kTcStageBytes, b0 = a0 + kTcABytes;
 #pragma unroll
@@ -229,6 +237,7 @@ __device__ __forceinline__ void conv_tile(const CUtensorMap& mapA, const CUtenso
                          smem_u32(kt + 1 < nk ? &empty[s] : &done))
                      : "memory");   // the last covers every instruction before it
       }
+      if (__builtin_expect(kt < nk, 0)) drain_instructions(&drain, &failed, err);
     }
     __syncwarp();
   }
@@ -237,8 +246,7 @@ __device__ __forceinline__ void conv_tile(const CUtensorMap& mapA, const CUtenso
     failed = 1;
     atomicExch(err, 1);
   }
-  if (!ok && tid == 0)   // the copies in flight, of slices that no instruction has waited for
-    for (int i = kt > ns ? kt - ns : 0; i < kt; i++) mbar_wait(&full[i % ns], (i / ns) & 1, &failed, false);
+  if (__builtin_expect(!ok && tid == 0, 0)) drain_copies(full, issued, &failed);
   __syncwarp();
   asm volatile("tcgen05.fence::after_thread_sync;");
   if (__all_sync(0xffffffffu, ok)) {
