@@ -22,7 +22,7 @@
 //
 // The slab form (k_xpass_adj3: 20 rows and 16 products of unpacked transforms,
 // one block per SM, products chosen by a switch at every point) took 574 us a
-// launch at 128x64x128; this 87 us. The whole adjoint step (us): 128x64x128
+// launch at 128x64x128; this 60 us. The whole adjoint step (us): 128x64x128
 // 1774 -> 362, 256x64x128 3829 -> 605, 256x1x256 222 -> 137, 64x1x64 134 -> 93.
 #include "sf_xmt.cuh"
 

@@ -63,10 +63,10 @@ struct ConvGemm {
 // instruction's transpose bits), as the tensors have them.
 //
 // Bound by the operands' way from L2: 24 KB a slice and SM, which takes about
-// 790 cycles on 104 SMs at once (6.1 TB/s over the GPU) against the
+// 840 cycles on 104 SMs at once (6.0 TB/s over the GPU) against the
 // instructions' 128; four slices in flight per CTA, two CTAs per SM (eight
 // slices measured the same). Measured, 13 samples of 256 levels: 1024 -> 256
-// channels forward 32 us, the 11 GEMMs of one gradient 0.18 ms in 8 launches,
+// channels forward 34 us under ncu, the 11 GEMMs of one gradient 0.18 ms in 8 launches,
 // where the version that gathered operands through registers took 3.29 ms.
 //
 // The K slices, and the runs of 16 of an instruction within them, go in the

@@ -20,7 +20,7 @@
 // transposes, the level below and the staged input rows. No block-wide barrier
 // after set-up: the groups of a warp march in step, warps are independent.
 //
-// The shared-memory pipe bounds it (82 to 89 % busy at 256x128x384). So the
+// The shared-memory pipe bounds it (81 % busy at 256x128x384). So the
 // nonlinear step carries its combinations in registers where a lane keeps three
 // modes or fewer, and forms the first batch of products from the inverse
 // transform's own registers: 230 us a stage with both in shared memory, 208
@@ -68,7 +68,7 @@ static void xmarch_launch(const StageArgs& a, int nruns, int t_lo, int t_hi, cud
 // shape here. 2D: where the slab kernel's blocks do not spread a few levels over
 // more SMs, from 2^17 points of the launch's runs, 2^13 at N1 = 128, whose rows
 // march two to a warp at 8 points a lane; always in mode 1, whose slabs copy the base's
-// rows as well. Measured, a whole step (us), slab and march:
+// rows as well. Near 2^17 points the two are even. Measured, a whole step (us), slab and march:
 //   N1 = 128      64 levels 37.8 36.9; 128 levels 47.1 45.1; 4 x 256 76.7 72.4; 1 + 2 tangents, 128 levels 83.4 73.8
 //   others        64x64 32.8 34.9; 256x64 36.9 38.9; 64x64 x 4 33.8 36.9; 256x128 47.1 49.5; 64x128 x 8 45.1 46.0;
 //                 256x256 x 2 75.8 75.8; 256x256 x 3 79.9 80.7; 512x388 110.9 107.6; 32x256 x 16 71.7 69.7

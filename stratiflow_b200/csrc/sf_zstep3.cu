@@ -38,9 +38,11 @@ constexpr ZfKernel zf_kernel() {
 //       two      2 x 128x64x180  46 (84.5), one 55.4;      256x128x128 67 (72.7), one 89.4
 //   2D  short4   64x1x64         10.2 (26.1)
 //       short8   128x1x128       12.4 (32.7), one 16.7;    32 x 128x1x128 19.8 (32.7), many 26.3
-//       one      6 x 512x1x388   26.9 (61.5), many 43.5;   64 x 256x1x384 130 (143), many 188
+//       one      6 x 512x1x388   26.9 (61.5), many 43.5, tall 27.4;  1 x 256x1x260 23.5, tall 25.5
 //       many     64 x 256x1x256  89.3 (101), one 99.8;     8 x 512x1x256 32.5 (40.5), one 36.3
-//       tall     as "one" where its columns do not fit: 64 x 256x1x384 125
+//       tall     as "one" where its columns do not fit. Over several waves of blocks of 384 levels
+//                and more it would be the faster: 64 x 256x1x384 127, one 135 (143); 32 x 256x1x484
+//                93, one 98; 16 x 256x1x388 49, one 48
 // Two blocks of an SM only pay where the SM's L1 keeps some of its room and
 // the second block has something to do; with one block each lane may hold
 // more levels' loads in flight.
