@@ -1119,8 +1119,12 @@ int sf_ensemble_step(sf_ensemble* e, int nsteps) {
   }
   // the stage arguments of every member for both parities (h, factors and
   // pointers may have changed since the last call); the graphs read them
-  // from the device table, which is written when they did
-  bool changed = !e->args_set;
+  // from the device table, which is written when they did, and again after a
+  // write that failed or was only recorded (the stream is being captured)
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  CK(cudaStreamIsCapturing(e->st, &capture));
+  const bool recorded = capture != cudaStreamCaptureStatusNone;
+  bool changed = !e->args_set || recorded;
   for (int p = 0; p < 2; p++)
     for (int k = 0; k < 3; k++) {
       const int cur = (k == 1) ? 1 - p : p;
@@ -1135,9 +1139,10 @@ int sf_ensemble_step(sf_ensemble* e, int nsteps) {
       }
     }
   if (changed) {
+    e->args_set = false;
     CK(cudaMemcpyAsync(e->d_args, e->h_args.data(), sizeof(StageArgs) * e->h_args.size(), cudaMemcpyHostToDevice,
                        e->st));
-    e->args_set = true;
+    e->args_set = !recorded;
   }
   for (int p = 0; p < 2; p++) {
     if (e->graph[p]) continue;
