@@ -383,12 +383,11 @@ int sf_net_gradient(sf_net* n, float* grad, double* loss);
  * (may be NULL) is the loss before step s */
 int sf_net_train(sf_net* n, int steps, double lr, double* losses);
 
-/* host memory for results (no counterpart in the reference): a block handed
- * to sf_net_forward or sf_net_gradient as the result's address is filled by
- * one direct copy at the link's rate. To everything else it is ordinary
- * memory: a copy from it that a program queues has read it when the call
- * returns, it outlives a reset of the device, and a forked child has a copy
- * of its own. */
+/* host memory (no counterpart in the reference) that sf_net_forward's and
+ * sf_net_gradient's results and sf_step_host_async's states are copied to, and
+ * from, at the link's rate. To every other call it is ordinary memory: a copy
+ * from it that a program queues has read it when the call returns, it outlives
+ * a reset of the device, and a forked child has a copy of its own. */
 int sf_host_alloc(size_t bytes, void** ptr);
 int sf_host_free(void* ptr);
 

@@ -86,12 +86,16 @@ void after_fork_child() {
 
 }  // namespace
 
-// where a copy of a result to p goes: the registered view of a block that starts there
-void* sf_host_dma(void* p) {
+// where the library's copies to and from p go: the registered view of a block that holds p
+void* sf_host_dma(const void* p) {
   Blocks& b = blocks();
+  char* c = static_cast<char*>(const_cast<void*>(p));
   std::lock_guard<std::mutex> lock(b.mu);
-  const auto it = b.by_view.find(p);
-  return it == b.by_view.end() ? p : it->second.dma;
+  auto it = b.by_view.upper_bound(c);
+  if (it == b.by_view.begin()) return c;
+  --it;
+  const size_t off = (size_t)(c - static_cast<char*>(it->first));
+  return off < it->second.bytes ? static_cast<char*>(it->second.dma) + off : c;
 }
 
 extern "C" {

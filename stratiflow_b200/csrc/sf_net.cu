@@ -28,7 +28,7 @@
 #include "../../include/stratiflow_b200.h"
 
 extern void sf_set_error_message(const std::string& msg);
-extern void* sf_host_dma(void* p);
+extern void* sf_host_dma(const void* p);
 
 namespace {
 

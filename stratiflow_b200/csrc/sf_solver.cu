@@ -311,6 +311,7 @@ const std::vector<double>& sf_solver_z(const sf_solver* s, int which) { return w
 const float2* sf_solver_tw(const sf_solver* s) { return s->tw; }
 const float* sf_solver_ubar(const sf_solver* s, int run) { return s->Ubar + (size_t)run * s->g.N3; }
 void sf_solver_count_launches(sf_solver* s, int n) { s->launches += n; }
+extern void* sf_host_dma(const void* p);
 
 extern "C" {
 
@@ -648,7 +649,7 @@ int sf_step_host_async(sf_solver* s, const float* host_in, float* host_out, int 
   const int b = (int)(P.k & 1);
   // the input, once the call two back has taken staging buffer b into its state
   CK(cudaStreamWaitEvent(P.h2d, P.ev_used[b], 0));
-  CK(cudaMemcpyAsync(P.in[b], host_in, bytes, cudaMemcpyHostToDevice, P.h2d));
+  CK(cudaMemcpyAsync(P.in[b], sf_host_dma(host_in), bytes, cudaMemcpyHostToDevice, P.h2d));
   CK(cudaEventRecord(P.ev_in[b], P.h2d));
   CK(cudaStreamWaitEvent(s->st, P.ev_in[b], 0));
   CK(cudaMemcpyAsync(s->S[s->cur], P.in[b], bytes, cudaMemcpyDeviceToDevice, s->st));
@@ -660,7 +661,7 @@ int sf_step_host_async(sf_solver* s, const float* host_in, float* host_out, int 
   CK(cudaMemcpyAsync(P.out[b], s->S[s->cur], bytes, cudaMemcpyDeviceToDevice, s->st));
   CK(cudaEventRecord(P.ev_done[b], s->st));
   CK(cudaStreamWaitEvent(P.d2h, P.ev_done[b], 0));
-  CK(cudaMemcpyAsync(host_out, P.out[b], bytes, cudaMemcpyDeviceToHost, P.d2h));
+  CK(cudaMemcpyAsync(sf_host_dma(host_out), P.out[b], bytes, cudaMemcpyDeviceToHost, P.d2h));
   CK(cudaEventRecord(P.ev_drained[b], P.d2h));
   P.k++;
   return SF_OK;

@@ -91,3 +91,36 @@ def test_results_outlive_a_reset_of_the_device():
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     r = subprocess.run([sys.executable, "-c", RESET], cwd=root, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and r.stdout.strip() == "same", r.stdout + r.stderr
+
+
+def test_states_stream_through_blocks():
+    """sf_step_host_async in and out of two states inside blocks of
+    sf_host_alloc, against the same states in arrays."""
+    import ctypes as C
+    import stratiflow_b200 as sf
+    from tests.helpers import CONFIGS, make_ic
+    from tests.test_gpu_parity import gpu_solver
+    s = gpu_solver(CONFIGS["kh2d"])
+    want, ins = [], []
+    for k in range(2):
+        s.set_state(0, make_ic(CONFIGS["kh2d"], seed=80 + k, amp=5e-2))
+        s.Prepare()
+        ins.append(s.get_state_kept())
+        s.TimeStep(2)
+        s.synchronize()
+        want.append(s.get_state_kept())
+    L, n, ptrs, bufs = sf.load_library(), ins[0].nbytes, [], []
+    for _ in range(2):
+        p = C.c_void_p()
+        assert L.sf_host_alloc(2 * n, C.byref(p)) == 0
+        ptrs.append(p)
+        bufs.append(np.frombuffer((C.c_char * (2 * n)).from_address(p.value), dtype=np.complex64)
+                    .reshape((2,) + s.kept_shape))
+    bufs[0][0], bufs[0][1] = ins
+    for k in range(2):
+        s.step_host_async(bufs[0][k], bufs[1][k], 2)
+    s.synchronize()
+    assert np.array_equal(bufs[1][0], want[0]) and np.array_equal(bufs[1][1], want[1])
+    del bufs
+    for p in ptrs:
+        assert L.sf_host_free(p) == 0
